@@ -1,10 +1,11 @@
 // Device kernels of the LocVolCalib engine (sm_100a).
 //
-//   lvc_setup_kernel    initGrid + initOperator + the strike-independent
-//                       per-step tables (finpar/LocVolCalib.fut:12-44, :50-66)
-//                       and the Y-direction LU pivots of every step.
-//   lvc_pivot_kernel    the X-direction LU pivots 1/b'_i of every (step, row)
-//                       (recurrence 1 of tridagPar, :71-91), strike-independent.
+//   lvc_setup_kernel    initGrid + initOperator: the strike-independent column,
+//                       row and step tables (finpar/LocVolCalib.fut:12-44).
+//   lvc_pivot_kernel    the rest of updateParams (:50-66) and the LU pivots of
+//                       every step (recurrence 1 of tridagPar, :71-91): 1/b'_i
+//                       of every (step, row) in X, 1/b'_j and the multipliers
+//                       of every step in Y; strike-independent.
 //   lvc_rollback_kernel persistent: one CTA (or a thread-block cluster) per
 //                       strike instance, the whole numY x numX grid resident in
 //                       shared memory for all numT-1 steps; each step is
@@ -22,9 +23,10 @@ namespace lvc {
 namespace cg = cooperative_groups;
 
 // ---------------------------------------------------------------------------
-// setup kernel: one CTA per calibration.  The grid and stencil formulas use
-// explicitly rounded operations (no FMA contraction) so the tables are the
-// reference's IEEE f64 values.
+// setup kernel: one CTA per calibration, the tables that depend on a column, a
+// row or a step alone.  The grid and stencil formulas use explicitly rounded
+// operations (no FMA contraction) so the tables are the reference's IEEE f64
+// values.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double grid_pt(int i, double d, double idx, double base) {
   // f32.i64 i * d - f32.i32 index * d + base   (:21-22)
@@ -60,7 +62,6 @@ __global__ void __launch_bounds__(256) lvc_setup_kernel(const CalibDev* __restri
   const double dy = __ddiv_rn(stdY, (double)Y);
   const double xidx = (double)c.xindex, yidx = (double)c.yindex;
   const double half_nu2 = __dmul_rn(0.5, __dmul_rn(c.nu, c.nu));  // 0.5 * var, var = nu*nu
-  const double half_nu_nu = __dmul_rn(__dmul_rn(0.5, c.nu), c.nu);  // 0.5 * nu * nu
 
   // Column tables: eX_i and 0.5 * Dxx_i[k]  (updateParams :63, explicitMethod :138-144)
   for (int i = tid; i < Xp; i += nt) {
@@ -109,168 +110,252 @@ __global__ void __launch_bounds__(256) lvc_setup_kernel(const CalibDev* __restri
   }
   const int steps = T > 1 ? T - 1 : 0;
   const double tden = __dsub_rn((double)T, 1.0);
-  // timeline t_k = t * k / (numT - 1) (:14), dtInv (:193), exp(2(y_j - 0.5 nu^2 t_k))
+  // timeline t_k = t * k / (numT - 1) (:14), dtInv (:193)
   for (int k = tid; k < steps; k += nt) {
     const double tn = __ddiv_rn(__dmul_rn(c.t, (double)k), tden);
     const double tx = __ddiv_rn(__dmul_rn(c.t, (double)(k + 1)), tden);
     tab[L.dtinv + k] = __ddiv_rn(1.0, __dsub_rn(tx, tn));
   }
-  for (int64_t e = tid; e < (int64_t)steps * Y; e += nt) {
-    const int k = (int)(e / Y), j = (int)(e % Y);
-    const double tn = __ddiv_rn(__dmul_rn(c.t, (double)k), tden);
-    const double yj = grid_pt(j, dy, yidx, logAlpha);
-    const double ev = exp(__dmul_rn(2.0, __dsub_rn(yj, __dmul_rn(half_nu_nu, tn))));
-    if (line)
-      tab[L.stab + ((int64_t)k * Y + j) * 8] = ev;
-    else
-      tab[L.eyt + (int64_t)k * L.eyt_ld + j] = ev;
-  }
-  __syncthreads();  // row tables and dtInv are visible to the whole CTA
+}
 
-  // Y-direction pivots of every step (implicitY: one matrix per step, shared
-  // by every column and every strike): b'_j = b_j - a_j c_{j-1} / b'_{j-1}.
-  for (int k = tid; k < steps; k += nt) {
-    const double dt = tab[L.dtinv + k];
-    double rb_prev = 0.0, c_prev = 0.0;
-    double* yc = line ? tab + L.stab + 8LL * k * Y : tab + L.yco + 4LL * k * Y;
-    const int w = line ? 8 : 4, o = line ? 1 : 0;
-    for (int j = 0; j < Y; j++) {
+// ---------------------------------------------------------------------------
+// pivot kernel: the pivot recurrences of both directions, written as 1/b', and
+// the per-step row tables.  A warp takes a group of recurrences of one
+// calibration, a lane each:
+//   Y groups (first) -- lane = one time step, walking the rows: the implicit-Y
+//     matrix is the same for every column and strike;
+//   X groups -- lane = one (step, row), walking the columns.
+//
+// With one calibration there are few warps, and a lane's chain is a division
+// and a multiply-add per element (74 cycles, 10 us for 256 elements), so all
+// else is kept off it: the coefficients of the next 16 or 32 elements come
+// through shared memory, loaded a block ahead, and groups go to as many SMs as
+// there are (warp w of CTA i takes group i + w * CTAs), because a warp's stores
+// are spread over 32 rows of memory: the Y groups of 255 steps x 256 rows write
+// 4.2 MB, which took 95 us from two SMs and X groups of 32 x 63 rows of 256
+// columns 75 us from 16.  For the same reason a Y group is 4 steps, not 32.
+// Setup and pivots together: 560 -> 46 us at 32 x 256 x 255 steps, 100 -> 38 us
+// at 256 x 32 x 63, and 4.0 ms of the 512-calibration mix's 254 ms, where 1.25e9
+// divisions and 10 GB of pivots are the bound (1.6 ms at the HBM rate).
+// ---------------------------------------------------------------------------
+constexpr int kPivotWarps = 4;  // warps per CTA (128 threads)
+constexpr int kYSteps = 4;      // time steps of a Y group
+constexpr int kPivotCols = 32;  // columns of an X warp's tile
+
+// Groups of one calibration's Y and X recurrences.
+LVC_HD int64_t y_groups(int T) { return T > 1 ? (T - 1 + kYSteps - 1) / kYSteps : 0; }
+LVC_HD int64_t x_groups(int Y, int T) { return T > 1 ? ((int64_t)(T - 1) * Y + 31) / 32 : 0; }
+
+// Last c in [0, ncal) with start[c] <= v.
+__device__ __forceinline__ int find_calib(const int64_t* __restrict__ start, int ncal, int64_t v) {
+  int lo = 0, hi = ncal - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (start[mid] <= v) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+// The Y recurrences of steps k0 .. k0 + kYSteps - 1 of calibration c (one lane
+// each): b'_j = b_j - a_j c_{j-1} / b'_{j-1}, the multipliers mY, nY and, for
+// the line family, their products inside each kLineK-row chunk of each CTA's row
+// block: cp_j = prod_{chunk start..j} mY, cq_j = prod_{j..chunk end} nY.
+// co: [kLineK][4] shared memory of this warp.
+__device__ __forceinline__ void y_pivots(const CalibDev& c, int k0, double* __restrict__ tabs, double (*co)[4]) {
+  const int lane = threadIdx.x & 31;
+  const int Y = c.numY, steps = c.numT - 1;
+  const bool line = c.kind == kKindLine;
+  const TabLayout L = tab_layout(c.numX, Y, c.numT, c.Xp, c.kind);
+  double* tab = tabs + c.tab;
+  const int k = k0 + lane;
+  const bool on = lane < kYSteps && k < steps;
+  const double dt = on ? tab[L.dtinv + k] : 1.0;
+  double* yc = tab + (line ? L.stab + 8LL * k * Y : L.yco + 4LL * k * Y);
+  double rb = 0.0;
+  int jb = 0, blk_end = min(Y, c.Ycs);  // chunk start, end of the CTA row block it lies in
+  while (jb < Y) {
+    const int n = min(kLineK, (line ? blk_end : Y) - jb);
+    // coefficients of the chunk's rows, a lane per row: a c_{j-1}, 0.5 g1, a, c
+    __syncwarp();
+    if (lane < n) {
+      const int j = jb + lane;
       const double* rc = tab + L.rowc + 4LL * j;
-      const double a = -(0.5 * rc[0]);
-      const double b = dt - 0.5 * rc[1];
-      const double cc = -(0.5 * rc[2]);
-      const double bp = (j == 0) ? b : b - a * c_prev * rb_prev;
-      const double rb = 1.0 / bp;
-      yc[w * j + o + 0] = (j == 0) ? 0.0 : -a * rb_prev;  // forward multiplier -a_j / b'_{j-1}
-      yc[w * j + o + 1] = (j == Y - 1) ? 0.0 : -cc * rb;  // backward multiplier -c_j / b'_j
-      yc[w * j + o + 2] = rb;
-      if (!line) yc[w * j + 3] = 0.0;
-      rb_prev = rb;
-      c_prev = cc;
+      const double a = -(0.5 * rc[0]), cc = -(0.5 * rc[2]);
+      const double cprev = j > 0 ? -(0.5 * rc[-2]) : 0.0;
+      co[lane][0] = a * cprev;
+      co[lane][1] = 0.5 * rc[1];
+      co[lane][2] = a;
+      co[lane][3] = j == Y - 1 ? 0.0 : cc;
     }
-    if (line) {
-      // products of the multipliers inside each kLineK-row chunk of each
-      // CTA's row block: cp_j = prod_{chunk start..j} mY, cq_j = prod_{j..chunk end} nY
-      for (int r0 = 0; r0 < Y; r0 += c.Ycs) {
-        const int r1 = min(Y, r0 + c.Ycs);
-        for (int jb = r0; jb < r1; jb += kLineK) {
-          const int je = min(r1, jb + kLineK);
-          double pr = 1.0;
-          for (int j = jb; j < je; j++) {
-            pr = pr * yc[8 * j + kSlotMY];
-            yc[8 * j + kSlotCP] = pr;
-          }
-          pr = 1.0;
-          for (int j = je - 1; j >= jb; j--) {
-            pr = pr * yc[8 * j + kSlotNY];
-            yc[8 * j + kSlotCQ] = pr;
-          }
-          for (int j = jb; j < je; j++) {
-            yc[8 * j + 5] = 0.0;
-            yc[8 * j + 7] = 0.0;
+    __syncwarp();
+    if (n == kLineK) {
+      double nY[kLineK], pr = 1.0;
+#pragma unroll
+      for (int m = 0; m < kLineK; m++) {
+        const double bp = (dt - co[m][1]) - co[m][0] * rb;
+        const double mY = -co[m][2] * rb;
+        rb = 1.0 / bp;
+        nY[m] = -co[m][3] * rb;
+        pr = pr * mY;
+        if (on) {
+          double* o = yc + (line ? 8LL : 4LL) * (jb + m);
+          if (line) {
+            o[kSlotMY] = mY;
+            *reinterpret_cast<double2*>(o + kSlotNY) = make_double2(nY[m], rb);
+            *reinterpret_cast<double2*>(o + kSlotCP) = make_double2(pr, 0.0);
+          } else {
+            reinterpret_cast<double2*>(o)[0] = make_double2(mY, nY[m]);
+            reinterpret_cast<double2*>(o)[1] = make_double2(rb, 0.0);
           }
         }
       }
+      if (line && on) {
+        pr = 1.0;
+#pragma unroll
+        for (int m = kLineK - 1; m >= 0; m--) {
+          pr = pr * nY[m];
+          *reinterpret_cast<double2*>(yc + 8LL * (jb + m) + kSlotCQ) = make_double2(pr, 0.0);
+        }
+      }
+    } else {  // the last rows of a block
+      double pr = 1.0;
+      for (int m = 0; m < n; m++) {
+        const double bp = (dt - co[m][1]) - co[m][0] * rb;
+        const double mY = -co[m][2] * rb;
+        rb = 1.0 / bp;
+        pr = pr * mY;
+        if (on) {
+          double* o = yc + (line ? 8LL : 4LL) * (jb + m);
+          if (line) {
+            o[kSlotMY] = mY;
+            *reinterpret_cast<double2*>(o + kSlotNY) = make_double2(-co[m][3] * rb, rb);
+            *reinterpret_cast<double2*>(o + kSlotCP) = make_double2(pr, 0.0);
+          } else {
+            reinterpret_cast<double2*>(o)[0] = make_double2(mY, -co[m][3] * rb);
+            reinterpret_cast<double2*>(o)[1] = make_double2(rb, 0.0);
+          }
+        }
+      }
+      if (line && on) {
+        pr = 1.0;
+        for (int m = n - 1; m >= 0; m--) {
+          double* o = yc + 8LL * (jb + m);
+          pr = pr * o[kSlotNY];
+          *reinterpret_cast<double2*>(o + kSlotCQ) = make_double2(pr, 0.0);
+        }
+      }
+    }
+    jb += n;
+    if (jb == blk_end) blk_end = min(Y, blk_end + c.Ycs);
+  }
+}
+
+// The X recurrences of rows r0 .. r0 + 31 of calibration c, row = step * numY +
+// row of the grid (one lane each), and those rows' e_j.  co, tile: shared
+// memory of this warp.
+template <typename PV>
+__device__ __forceinline__ void x_pivots(const CalibDev& c, int64_t r0, double* __restrict__ tabs,
+                                         PV* __restrict__ piv, double (*co)[4], double (*tile)[kPivotCols + 1]) {
+  const int lane = threadIdx.x & 31;
+  const int X = c.numX, Y = c.numY;
+  const bool line = c.kind == kKindLine;
+  const TabLayout L = tab_layout(X, Y, c.numT, c.Xp, c.kind);
+  double* tab = tabs + c.tab;
+  const int64_t rows = (int64_t)(c.numT - 1) * Y;
+  const int nr = (int)min((int64_t)32, rows - r0);  // rows of this group
+  const int64_t r = min(r0 + lane, rows - 1);
+  const int k = (int)(r / Y), j = (int)(r - (int64_t)k * Y);
+  const double dt = tab[L.dtinv + k];
+  // line family: the line kernels' shared-memory image of a row, stride ld
+  const int LD = line ? c.ld : c.Xp;
+  PV* const row = piv + c.piv + ((int64_t)k * (line ? round4(Y) : Y) + j) * LD;
+  // a block's coefficients, a lane per column: W0, W1, W2 (line) or 0.5 Dxx, eX
+  double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
+  auto fetch = [&](int i) {
+    if (i >= X) return;
+    if (line) {
+      v0 = tab[L.wcol + i];
+      v1 = tab[L.wcol + L.xa + i];
+      v2 = tab[L.wcol + 2 * L.xa + i];
+    } else {
+      const double2 c01 = *reinterpret_cast<const double2*>(tab + L.colc + 4LL * i);
+      const double2 c23 = *reinterpret_cast<const double2*>(tab + L.colc + 4LL * i + 2);
+      v0 = c01.y;
+      v1 = c23.x;
+      v2 = c23.y;
+      v3 = c01.x;
+    }
+  };
+  fetch(lane);
+  // e_j of the step: exp(2 (y_j - 0.5 nu^2 t_k))  (updateParams, :63)
+  const double tn = __ddiv_rn(__dmul_rn(c.t, (double)k), __dsub_rn((double)c.numT, 1.0));
+  const double dy = __ddiv_rn(__dmul_rn(__dmul_rn(10.0, c.nu), sqrt(c.t)), (double)Y);
+  const double yj = grid_pt(j, dy, (double)c.yindex, log(c.alpha));
+  const double e = exp(__dmul_rn(2.0, __dsub_rn(yj, __dmul_rn(__dmul_rn(__dmul_rn(0.5, c.nu), c.nu), tn))));
+  if (lane < nr) tab[line ? L.stab + ((int64_t)k * Y + j) * 8 + kSlotE : L.eyt + (int64_t)k * L.eyt_ld + j] = e;
+  double rb = 0.0, c_prev = 0.0;  // 1/b' and c of the column before: zero before the first
+  for (int c0 = 0; c0 < LD; c0 += kPivotCols) {
+    __syncwarp();
+    co[lane][0] = v0;
+    co[lane][1] = v1;
+    co[lane][2] = v2;
+    co[lane][3] = v3;
+    __syncwarp();
+    fetch(c0 + kPivotCols + lane);
+    const int n = min(kPivotCols, X - c0);
+#pragma unroll 8
+    for (int m = 0; m < n; m++) {
+      double a, b, cc;
+      if (line) {
+        // b'_i = (dt - e W1_i) - (e W0_i)(e W2_{i-1}) / b'_{i-1}
+        a = -(e * co[m][0]);
+        b = dt - e * co[m][1];
+        cc = -(e * co[m][2]);
+      } else {
+        const double var = co[m][3] * e;
+        a = -(0.5 * (var * co[m][0]));
+        b = dt - 0.5 * (var * co[m][1]);
+        cc = -(0.5 * (var * co[m][2]));
+      }
+      rb = 1.0 / (b - a * c_prev * rb);
+      c_prev = cc;
+      tile[lane][m] = rb;
+    }
+    for (int m = max(n, 0); m < kPivotCols; m++) tile[lane][m] = 0.0;  // padding columns
+    __syncwarp();
+    const bool w = c0 + lane < LD;
+    auto put = [&](int q) {
+      PV* o = reinterpret_cast<PV*>(__shfl_sync(0xffffffffu, (unsigned long long)row, q));
+      if (w) o[c0 + lane] = (PV)tile[q][lane];
+    };
+    if (nr == 32) {
+#pragma unroll 8
+      for (int q = 0; q < 32; q++) put(q);
+    } else {
+      for (int q = 0; q < nr; q++) put(q);
     }
   }
 }
 
-// ---------------------------------------------------------------------------
-// pivot kernel: one lane per (calibration, step, row) runs the sequential pivot
-// recurrence of one X-direction system, written as 1/b'_i.  A warp owns 32
-// consecutive rows and goes through them 32 columns at a time: every lane
-// puts its 32 pivots in a shared tile, then the warp writes the tile out one
-// row at a time, 32 consecutive columns per store, so every row leaves in
-// whole 32-byte sectors (a store per lane per column would touch 32 rows per
-// instruction and leave partly written sectors to the L2).
-// ---------------------------------------------------------------------------
-constexpr int kPivotWarps = 4;  // warps per CTA (128 threads)
-
+// starts: [2][ncal + 1] prefix sums over the calibrations of y_groups() and of
+// x_groups().
 template <typename PV>
-__global__ void __launch_bounds__(128) lvc_pivot_kernel(const CalibDev* __restrict__ calibs,
-                                                        const int64_t* __restrict__ row_start,
-                                                        int ncal, const double* __restrict__ tabs,
-                                                        PV* __restrict__ piv) {
-  __shared__ double tile[kPivotWarps][32][33];
-  __shared__ PV* rowp[kPivotWarps][32];
-  __shared__ int rowx[kPivotWarps][32], rowld[kPivotWarps][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int64_t total = row_start[ncal];
-  const int64_t ngroups = (total + 31) / 32;
-  for (int64_t g = (int64_t)blockIdx.x * kPivotWarps + w; g < ngroups; g += (int64_t)gridDim.x * kPivotWarps) {
-    const int64_t r = g * 32 + lane;
-    int X = 0, LDr = 0;
-    PV* o = nullptr;
-    bool line = false;
-    double e = 0.0, dt = 0.0;
-    const double* tab = tabs;
-    TabLayout L{};
-    if (r < total) {
-      int lo = 0, hi = ncal - 1;  // last c with row_start[c] <= r
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (row_start[mid] <= r) lo = mid; else hi = mid - 1;
-      }
-      const CalibDev c = calibs[lo];
-      const int Y = c.numY;
-      X = c.numX;
-      L = tab_layout(X, Y, c.numT, c.Xp, c.kind);
-      const int64_t local = r - row_start[lo];
-      const int k = (int)(local / Y), j = (int)(local % Y);
-      tab = tabs + c.tab;
-      dt = tab[L.dtinv + k];
-      line = c.kind == kKindLine;
-      if (line) {
-        // rows of stride ld: the line kernels' shared-memory image
-        e = tab[L.stab + ((int64_t)k * Y + j) * 8];
-        LDr = c.ld;
-        o = piv + c.piv + ((int64_t)k * round4(Y) + j) * LDr;
-      } else {
-        e = tab[L.eyt + (int64_t)k * L.eyt_ld + j];
-        LDr = c.Xp;
-        o = piv + c.piv + ((int64_t)k * Y + j) * LDr;
-      }
-    }
-    rowp[w][lane] = o;
-    rowx[w][lane] = X;
-    rowld[w][lane] = LDr;
-    const int maxld = __reduce_max_sync(0xffffffffu, (unsigned)LDr);
-    __syncwarp();
-    double rb_prev = 0.0, c_prev = 0.0;
-    for (int c0 = 0; c0 < maxld; c0 += 32) {
-      for (int m = 0; m < 32; m++) {
-        const int i = c0 + m;
-        double rb = 0.0;
-        if (i < X) {
-          double a, b, cc;
-          if (line) {
-            // b'_i = (dt - e W1_i) - (e W0_i)(e W2_{i-1}) / b'_{i-1}
-            const double* W0 = tab + L.wcol;
-            a = -(e * W0[i]);
-            b = dt - e * W0[L.xa + i];
-            cc = -(e * W0[2 * L.xa + i]);
-          } else {
-            const double2 c01 = *reinterpret_cast<const double2*>(tab + L.colc + 4LL * i);
-            const double2 c23 = *reinterpret_cast<const double2*>(tab + L.colc + 4LL * i + 2);
-            const double var = c01.x * e;
-            a = -(0.5 * (var * c01.y));
-            b = dt - 0.5 * (var * c23.x);
-            cc = -(0.5 * (var * c23.y));
-          }
-          const double bp = (i == 0) ? b : b - a * c_prev * rb_prev;
-          rb = 1.0 / bp;
-          rb_prev = rb;
-          c_prev = cc;
-        }
-        tile[w][lane][m] = rb;
-      }
-      __syncwarp();
-      for (int rr = 0; rr < 32; rr++) {
-        PV* orow = rowp[w][rr];
-        const int i = c0 + lane;
-        if (orow && i < rowld[w][rr]) orow[i] = (PV)(i < rowx[w][rr] ? tile[w][rr][lane] : 0.0);
-      }
-      __syncwarp();
+__global__ void __launch_bounds__(32 * kPivotWarps) lvc_pivot_kernel(const CalibDev* __restrict__ calibs,
+                                                                     const int64_t* __restrict__ starts, int ncal,
+                                                                     double* __restrict__ tabs,
+                                                                     PV* __restrict__ piv) {
+  __shared__ double tile[kPivotWarps][32][kPivotCols + 1];
+  __shared__ double co[kPivotWarps][32][4];
+  const int w = threadIdx.x >> 5;
+  const int64_t* xg_start = starts + ncal + 1;
+  const int64_t yg = starts[ncal], ngroups = yg + xg_start[ncal];
+  for (int64_t g = blockIdx.x + (int64_t)w * gridDim.x; g < ngroups; g += (int64_t)kPivotWarps * gridDim.x) {
+    if (g < yg) {
+      const int ci = find_calib(starts, ncal, g);
+      y_pivots(calibs[ci], (int)(g - starts[ci]) * kYSteps, tabs, co[w]);
+    } else {
+      const int ci = find_calib(xg_start, ncal, g - yg);
+      x_pivots<PV>(calibs[ci], (g - yg - xg_start[ci]) * 32, tabs, piv, co[w], tile[w]);
     }
   }
 }

@@ -295,13 +295,13 @@ struct lvc_plan {
   std::vector<Config> cfgs;  // the shape each calibration runs under
   std::vector<Launch> launches;
   std::vector<Item> items;
-  std::vector<int64_t> row_start;
+  std::vector<int64_t> starts;  // the pivot kernel's [2][ncal + 1]: y_groups(), x_groups()
   int64_t tab_elems = 0, piv_elems = 0, gstate_elems = 0;
   CalibDev* d_calibs = nullptr;
   double* d_tabs = nullptr;
   void* d_piv = nullptr;
   double* d_out = nullptr;
-  int64_t* d_rowstart = nullptr;
+  int64_t* d_starts = nullptr;
   Item* d_items = nullptr;
   void* d_gstate = nullptr;
   int* d_err = nullptr;
@@ -712,12 +712,12 @@ cudaError_t plan_enqueue(lvc_plan* P, cudaStream_t s, cudaEvent_t* ev) {
   if (P->ncal == 0) return cudaSuccess;
   lvc_setup_kernel<<<P->ncal, 256, 0, s>>>(P->d_calibs, P->d_tabs);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if (P->row_start.back() > 0) {
+  if (P->starts[P->ncal] > 0) {
     if (P->precision == LVC_F64)
-      lvc_pivot_kernel<double><<<P->pivot_grid, 128, 0, s>>>(P->d_calibs, P->d_rowstart, P->ncal,
+      lvc_pivot_kernel<double><<<P->pivot_grid, 128, 0, s>>>(P->d_calibs, P->d_starts, P->ncal,
                                                               P->d_tabs, (double*)P->d_piv);
     else
-      lvc_pivot_kernel<float><<<P->pivot_grid, 128, 0, s>>>(P->d_calibs, P->d_rowstart, P->ncal,
+      lvc_pivot_kernel<float><<<P->pivot_grid, 128, 0, s>>>(P->d_calibs, P->d_starts, P->ncal,
                                                              P->d_tabs, (float*)P->d_piv);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
@@ -759,7 +759,7 @@ void plan_release(lvc_plan* P) {
   if (P->ev_fork) cudaEventDestroy(P->ev_fork);
   for (cudaEvent_t e : P->ev_join)
     if (e) cudaEventDestroy(e);
-  void* bufs[] = {P->d_calibs, P->d_tabs, P->d_piv, P->d_out, P->d_rowstart, P->d_items, P->d_gstate, P->d_err};
+  void* bufs[] = {P->d_calibs, P->d_tabs, P->d_piv, P->d_out, P->d_starts, P->d_items, P->d_gstate, P->d_err};
   for (void* b : bufs) {
     if (!b) continue;
     if (P->pool) P->pool->release(b); else cudaFree(b);
@@ -781,13 +781,21 @@ void fill_scalars(CalibDev& d, const lvc_calibration& c) {
   d.yindex = c.numY / 2;
 }
 
+// CTAs of the pivot kernel: one per group while that leaves no SM with more than
+// a full load of them (the groups then sit on as many SMs as there are).
+int pivot_grid(const futhark_context* ctx, int64_t groups) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(groups, 16LL * ctx->num_sms));
+}
+
 template <typename S, typename PV>
 int plan_build(futhark_context* ctx, const lvc_calibration* cs, int n, lvc_plan* P) {
   P->ncal = n;
   P->params.assign(cs, cs + n);
   P->calibs.resize(n);
   P->cfgs.resize(n);
-  P->row_start.assign(n + 1, 0);
+  P->starts.assign(2 * (n + 1), 0);
+  int64_t* const yg_start = P->starts.data();
+  int64_t* const xg_start = yg_start + n + 1;
   std::map<std::tuple<int, int, int, int, bool, bool, bool, int>, std::vector<std::pair<int64_t, Item>>> classes;
   std::map<std::tuple<int, int, int, int, bool, bool, bool, int>, Config> class_cfg;
   int64_t tab_off = 0, piv_off = 0, out_off = 0;
@@ -814,7 +822,8 @@ int plan_build(futhark_context* ctx, const lvc_calibration* cs, int n, lvc_plan*
     piv_off += (piv_elems(c.numX, c.numY, c.numT, d.Xp, d.kind, d.ld) + 3) & ~int64_t(3);
     d.out = out_off;
     out_off += c.outer;
-    P->row_start[i + 1] = P->row_start[i] + (int64_t)(c.numT > 1 ? c.numT - 1 : 0) * c.numY;
+    yg_start[i + 1] = yg_start[i] + y_groups(c.numT);
+    xg_start[i + 1] = xg_start[i] + x_groups(c.numY, c.numT);
     const auto key = std::make_tuple(cf.kind, cf.NT, cf.KX, cf.C, cf.gstate, cf.full, cf.pair, cf.upw);
     auto& cls = classes[key];
     auto it = class_cfg.find(key);
@@ -879,8 +888,7 @@ int plan_build(futhark_context* ctx, const lvc_calibration* cs, int n, lvc_plan*
     for (size_t i : ord) sorted.push_back(P->launches[i]);
     P->launches.swap(sorted);
   }
-  const int64_t rows = P->row_start[n];
-  P->pivot_grid = (int)std::max<int64_t>(1, std::min<int64_t>((rows + 127) / 128, 64LL * ctx->num_sms));
+  P->pivot_grid = pivot_grid(ctx, yg_start[n] + xg_start[n]);
 
   // device buffers
   auto dalloc = [&](void** dst, size_t bytes) -> int {
@@ -896,7 +904,7 @@ int plan_build(futhark_context* ctx, const lvc_calibration* cs, int n, lvc_plan*
   if (int rc = dalloc((void**)&P->d_tabs, sizeof(double) * std::max<int64_t>(2, P->tab_elems))) return rc;
   if (int rc = dalloc(&P->d_piv, sizeof(PV) * std::max<int64_t>(4, P->piv_elems))) return rc;
   if (int rc = dalloc((void**)&P->d_out, sizeof(double) * std::max<int64_t>(1, P->nprices))) return rc;
-  if (int rc = dalloc((void**)&P->d_rowstart, sizeof(int64_t) * (n + 1))) return rc;
+  if (int rc = dalloc((void**)&P->d_starts, sizeof(int64_t) * P->starts.size())) return rc;
   if (int rc = dalloc((void**)&P->d_items, sizeof(Item) * std::max<size_t>(1, P->items.size()))) return rc;
   if (P->gstate_elems > 0)
     if (int rc = dalloc(&P->d_gstate, sizeof(S) * P->gstate_elems)) return rc;
@@ -904,7 +912,7 @@ int plan_build(futhark_context* ctx, const lvc_calibration* cs, int n, lvc_plan*
   if (n > 0)
     LVC_CUDA(ctx, cudaMemcpyAsync(P->d_calibs, P->calibs.data(), sizeof(CalibDev) * n,
                                   cudaMemcpyHostToDevice, ctx->stream));
-  LVC_CUDA(ctx, cudaMemcpyAsync(P->d_rowstart, P->row_start.data(), sizeof(int64_t) * (n + 1),
+  LVC_CUDA(ctx, cudaMemcpyAsync(P->d_starts, P->starts.data(), sizeof(int64_t) * P->starts.size(),
                                 cudaMemcpyHostToDevice, ctx->stream));
   if (!P->items.empty())
     LVC_CUDA(ctx, cudaMemcpyAsync(P->d_items, P->items.data(), sizeof(Item) * P->items.size(),
@@ -1345,7 +1353,7 @@ const double* lvc_plan_device_prices(const struct lvc_plan* plan) { return plan 
 
 int32_t lvc_plan_num_launches(const struct lvc_plan* plan) {
   if (!plan || plan->ncal == 0) return 0;
-  int32_t n = 1 + (plan->row_start.back() > 0 ? 1 : 0);
+  int32_t n = 1 + (plan->starts[plan->ncal] > 0 ? 1 : 0);
   for (const auto& L : plan->launches) n += L.n_items > 0 ? 1 : 0;
   return n;
 }
@@ -1933,7 +1941,7 @@ size_t up256(size_t n) { return (n + 255) & ~size_t(255); }
 // The scratch carve-up of one call: calibration record, error flag, row
 // table, work list, operator tables and pivot rows, each on a 256-byte boundary.
 struct NoallocCarve {
-  size_t o_calib, o_err, o_rows, o_items, o_tabs, o_piv, need;
+  size_t o_calib, o_err, o_starts, o_items, o_tabs, o_piv, need;
 };
 NoallocCarve noalloc_carve(const Config& cf, int outer, int numX, int numY, int numT) {
   const int Xp = std::max(8, pow2ceil(numX));
@@ -1942,8 +1950,8 @@ NoallocCarve noalloc_carve(const Config& cf, int outer, int numX, int numY, int 
   NoallocCarve c;
   c.o_calib = 0;
   c.o_err = up256(c.o_calib + sizeof(CalibDev));
-  c.o_rows = up256(c.o_err + sizeof(int));
-  c.o_items = up256(c.o_rows + 2 * sizeof(int64_t));
+  c.o_starts = up256(c.o_err + sizeof(int));
+  c.o_items = up256(c.o_starts + 4 * sizeof(int64_t));
   c.o_tabs = up256(c.o_items + sizeof(Item) * (size_t)std::max(1, outer));
   c.o_piv = up256(c.o_tabs + sizeof(double) * (size_t)tab_elems);
   c.need = c.o_piv + sizeof(double) * (size_t)piv_n;
@@ -1995,7 +2003,7 @@ extern "C" int lvc_entry_main_f64_noalloc(struct futhark_context* ctx, double* p
   d.piv = 0;
   d.out = 0;
   const NoallocCarve cv = noalloc_carve(cf, outer, numX, numY, numT);
-  const size_t o_calib = cv.o_calib, o_err = cv.o_err, o_rows = cv.o_rows, o_items = cv.o_items,
+  const size_t o_calib = cv.o_calib, o_err = cv.o_err, o_starts = cv.o_starts, o_items = cv.o_items,
                o_tabs = cv.o_tabs, o_piv = cv.o_piv, need = cv.need;
   if (need > kNoAllocScratchBytes) {
     char buf[256];
@@ -2007,26 +2015,25 @@ extern "C" int lvc_entry_main_f64_noalloc(struct futhark_context* ctx, double* p
   }
   CalibDev* d_calib = reinterpret_cast<CalibDev*>(base + o_calib);
   int* d_err = reinterpret_cast<int*>(base + o_err);
-  int64_t* d_rows = reinterpret_cast<int64_t*>(base + o_rows);
+  int64_t* d_starts = reinterpret_cast<int64_t*>(base + o_starts);
   Item* d_items = reinterpret_cast<Item*>(base + o_items);
   double* d_tabs = reinterpret_cast<double*>(base + o_tabs);
   double* d_piv = reinterpret_cast<double*>(base + o_piv);
-  const int64_t rows[2] = {0, (int64_t)(numT > 1 ? numT - 1 : 0) * numY};
+  const int64_t starts[4] = {0, y_groups(numT), 0, x_groups(numY, numT)};
   cudaStream_t s = ctx->stream;
 
   // the array keeps the previous call's contents: reset what must start at zero
   LVC_CUDA(ctx, cudaMemsetAsync(d_err, 0, sizeof(int), s));
   LVC_CUDA(ctx, cudaMemcpyAsync(d_calib, &d, sizeof d, cudaMemcpyHostToDevice, s));
-  LVC_CUDA(ctx, cudaMemcpyAsync(d_rows, rows, sizeof rows, cudaMemcpyHostToDevice, s));
+  LVC_CUDA(ctx, cudaMemcpyAsync(d_starts, starts, sizeof starts, cudaMemcpyHostToDevice, s));
   if (outer > 0) {
     lvc_noalloc_items_kernel<<<(outer + 255) / 256, 256, 0, s>>>(d_items, outer);
     LVC_CUDA(ctx, cudaGetLastError());
   }
   lvc_setup_kernel<<<1, 256, 0, s>>>(d_calib, d_tabs);
   LVC_CUDA(ctx, cudaGetLastError());
-  if (rows[1] > 0) {
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((rows[1] + 127) / 128, 64LL * ctx->num_sms));
-    lvc_pivot_kernel<double><<<grid, 128, 0, s>>>(d_calib, d_rows, 1, d_tabs, d_piv);
+  if (starts[1] > 0) {
+    lvc_pivot_kernel<double><<<pivot_grid(ctx, starts[1] + starts[3]), 128, 0, s>>>(d_calib, d_starts, 1, d_tabs, d_piv);
     LVC_CUDA(ctx, cudaGetLastError());
   }
   if (outer > 0) {
