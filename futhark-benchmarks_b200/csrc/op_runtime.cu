@@ -542,153 +542,267 @@ __global__ void __launch_bounds__(kOpReduceThreads) op_reduce_kernel(const doubl
 // as its golden outputs were produced): an f32 running sum in path order,
 // s_k = fl(s_{k-1} + p_k).  Computed exactly, in parallel, from one fact: while
 // s stays in one binade [2^e, 2^(e+1)) -- f32 grid spacing u = 2^(e-23) -- and
-// p_k >= 0, fl(s + p_k) = s + u * t_k, where t_k is p_k / u rounded to the
-// nearest integer and does not depend on s (except on an exact tie, whose
-// round-to-even goes by the parity of s / u).  So a chunk of payoffs adds the
-// integer sum of its t_k to s / u until the sum would leave the binade; the
-// payoffs where that happens, ties, zero or tiny running sums and anything not
-// a finite nonnegative normal number are added one at a time in f32, exactly
-// as the sequential loop does.
+// 0 <= p_k < 2^e, fl(s + p_k) = s + u * t_k, where t_k is p_k / u rounded to the
+// nearest integer, and on a tie to the one that makes s / u even.  So payoffs
+// act on s / u as integer additions that depend on s through its parity alone,
+// and a run of them as a pair of additions, one per parity; such pairs compose.
+//
+//   op_seq_maps_kernel  a warp per block of kSeqBlock payoffs: the block's pair
+//                       for the exponent that the mean payoff (already known
+//                       from the f64 sum) predicts, or the two it lies between;
+//   op_seq_reduce_kernel  one CTA per model: composes the blocks' pairs from the
+//                       running sum on, up to the first block in which the sum
+//                       leaves its binade; that block's payoffs are added one
+//                       after the other in f32, as the sequential loop does (and
+//                       so is every block holding a payoff that is not a finite
+//                       nonnegative normal number below 2^e).
+//
+// The sum leaves its binade about once per doubling of the paths: for 8.4 M
+// payoffs 15 blocks are walked and 8 steps composed, one after the other, and
+// that chain's latency (4 us each: the pairs' and payoffs' loads from L2, two
+// scans, 256 additions) bounds the second kernel; the first is bound by its
+// instructions.  One CTA walking all payoffs 16384 at a time, as before, took
+// 7 us per step, 4.01 ms in all; now 26 + 105 us.
 // ---------------------------------------------------------------------------
+constexpr int kSeqBlock = 256;    // payoffs per block: 8 per lane of a warp
 constexpr int kSeqThreads = 1024;
-constexpr int kSeqPer = 16;  // payoffs per thread per chunk
+constexpr int kSeqPer = 4;        // blocks per thread and step of the composition
+constexpr int kSeqMaps = 2;       // exponents a block's pair is made for, at most
+constexpr uint32_t kSeqLim = 1u << 24;   // s / u reaching 2^24 leaves the binade
+constexpr uint32_t kSeqNone = 1u << 30;  // no pair: larger than any sum in the binade
 
-// t = p / 2^(e-23) rounded to nearest; false when p needs a step of its own
-// (a tie, p >= 2^e, p negative, non-finite or subnormal)
-__device__ __forceinline__ bool seq_units(float p, int e, uint32_t& t) {
+// What a run of payoffs adds to s / u, by the parity of s / u before it.
+struct SeqPair {
+  uint32_t a0, a1;
+};
+__device__ __forceinline__ uint32_t seq_cap(uint32_t v) { return min(v, kSeqNone); }
+// f, then g
+__device__ __forceinline__ SeqPair seq_then(SeqPair f, SeqPair g) {
+  return {seq_cap(f.a0 + ((f.a0 & 1u) ? g.a1 : g.a0)), seq_cap(f.a1 + ((f.a1 & 1u) ? g.a0 : g.a1))};
+}
+// The run a followed by payoff p, for sums in binade e; false when p needs a
+// step of its own in f32.
+__device__ __forceinline__ bool seq_add(SeqPair& a, float p, int e) {
   const uint32_t b = __float_as_uint(p);
-  if (b == 0u) {  // +0
-    t = 0;
-    return true;
-  }
-  const int be = (int)((b >> 23) & 0xffu);
-  if ((b >> 31) || be == 0 || be == 0xff) return false;
-  const int d = e - (be - 127);  // p in [2^(e-d), 2^(e-d+1))
-  if (d < 1) return false;
+  if (b == 0u) return true;  // +0
+  const int be = (int)(b >> 23);  // sign and exponent: above 0xfe is negative, infinite or NaN
+  const int d = e - (be - 127);   // p in [2^(e-d), 2^(e-d+1))
+  if (be == 0 || be > 0xfe || d < 1) return false;
   const uint32_t m = (b & 0x7fffffu) | 0x800000u;
-  if (d > 31) {
-    t = 0;
-    return true;
-  }
-  t = m >> d;
-  const uint32_t rem = m & ((1u << d) - 1u), half = 1u << (d - 1);
-  if (rem == half) return false;
-  t += rem > half;
+  const int sh = min(d, 26);  // beyond that p is less than half a unit, as at 26
+  const uint32_t t = m >> sh, rem = m & ((1u << sh) - 1u), half = 1u << (sh - 1);
+  const bool tie = rem == half;
+  const uint32_t up = rem > half;
+  a.a0 = seq_cap(a.a0 + t + (tie ? ((a.a0 + t) & 1u) : up));
+  a.a1 = seq_cap(a.a1 + t + (tie ? ((a.a1 + t + 1u) & 1u) : up));
   return true;
 }
 
-__device__ __forceinline__ int64_t warp_excl_scan(int64_t v, int lane) {
-  int64_t x = v;
+// The exponents block b's pairs are made for: those of the sum that the mean
+// payoff predicts before the block, give or take a quarter.
+__device__ __forceinline__ int seq_exponent(float s) { return (int)((__float_as_uint(s) >> 23) & 0xffu) - 127; }
+__device__ __forceinline__ void seq_exponents(float mean, int64_t b, int& lo, int& hi) {
+  const float s = mean * (float)(b * kSeqBlock);
+  lo = seq_exponent(s * 0.8f);
+  hi = seq_exponent(s * 1.25f);
+}
+
+// The pair of a block's payoffs for binade e, in every lane of the warp.
+__device__ __forceinline__ SeqPair seq_block_pair(const float (&v)[kSeqBlock / 32], int n, int e) {
+  constexpr int PL = kSeqBlock / 32;
+  const int lane = threadIdx.x & 31;
+  SeqPair a{0u, 0u};
+  bool ok = true;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
+  for (int j = 0; j < PL; j++)
+    if (lane * PL + j < n) ok = ok && seq_add(a, v[j], e);
+  if (!ok) a = {kSeqNone, kSeqNone};
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {  // lanes in order: lane l holds lanes l .. l + 2 o - 1
+    const SeqPair g{__shfl_down_sync(0xffffffffu, a.a0, o), __shfl_down_sync(0xffffffffu, a.a1, o)};
+    if ((lane & (2 * o - 1)) == 0) a = seq_then(a, g);
   }
-  return x - v;
+  return {__shfl_sync(0xffffffffu, a.a0, 0), __shfl_sync(0xffffffffu, a.a1, 0)};
+}
+// A block's payoffs, consecutive ones per lane; true when all are +0.
+__device__ __forceinline__ bool seq_load_block(const float* __restrict__ p, int num_models, int64_t b, int n,
+                                               float (&v)[kSeqBlock / 32]) {
+  constexpr int PL = kSeqBlock / 32;
+  static_assert(PL % 4 == 0, "16-byte loads");
+  const int lane = threadIdx.x & 31;
+  const float* q = p + (b * kSeqBlock + lane * PL) * num_models;
+  uint32_t any = 0;
+  if (num_models == 1 && n == kSeqBlock && ((uintptr_t)q & 15) == 0) {
+#pragma unroll
+    for (int j = 0; j < PL; j += 4) {
+      const float4 t = *reinterpret_cast<const float4*>(q + j);
+      v[j] = t.x;
+      v[j + 1] = t.y;
+      v[j + 2] = t.z;
+      v[j + 3] = t.w;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < PL; j++) v[j] = lane * PL + j < n ? q[(int64_t)j * num_models] : 0.0f;
+  }
+#pragma unroll
+  for (int j = 0; j < PL; j++) any |= __float_as_uint(v[j]);
+  return __all_sync(0xffffffffu, any == 0u);
+}
+
+// maps[mm][kSeqMaps][block].  A block of zeros has (0, 0) for every exponent,
+// written with kSeqZeros as the second number, so that it is known as one.
+constexpr uint32_t kSeqZeros = 0x80000000u;
+__global__ void __launch_bounds__(256) op_seq_maps_kernel(const float* __restrict__ pay, int64_t N, int num_models,
+                                                          int m0, const float* __restrict__ mean,
+                                                          SeqPair* __restrict__ maps) {
+  const int lane = threadIdx.x & 31, mm = blockIdx.y;
+  const int64_t blocks = (N + kSeqBlock - 1) / kSeqBlock;
+  const int64_t b = (int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+  if (b >= blocks) return;
+  const int n = (int)min((int64_t)kSeqBlock, N - b * kSeqBlock);
+  float v[kSeqBlock / 32];
+  const bool zeros = seq_load_block(pay + m0 + mm, num_models, b, n, v);
+  int lo, hi;
+  seq_exponents(mean[m0 + mm], b, lo, hi);
+  for (int e = lo; e <= hi; e++) {
+    SeqPair a{0u, kSeqZeros};
+    if (!zeros) a = seq_block_pair(v, n, e);
+    if (lane == 0) maps[((int64_t)mm * kSeqMaps + (e - lo)) * blocks + b] = a;
+  }
 }
 
 __global__ void __launch_bounds__(kSeqThreads) op_seq_reduce_kernel(const float* __restrict__ pay, int64_t N,
                                                                     int num_models, int m0, int num_mc_it,
+                                                                    const SeqPair* __restrict__ maps,
                                                                     float* __restrict__ out) {
+  constexpr int NW = kSeqThreads / 32;
   const int mm = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float* p = pay + m0 + mm;  // path k at p[k * num_models]
-  __shared__ float s_sum;
-  __shared__ long long s_next;
+  const int64_t blocks = (N + kSeqBlock - 1) / kSeqBlock;
+  const float mean = out[m0 + mm];
+  const SeqPair* mp = maps + (int64_t)mm * blocks * kSeqMaps;
+  __shared__ __align__(16) float s_pay[kSeqBlock];
+  __shared__ SeqPair s_warp[NW];
+  __shared__ uint32_t s_base;
   __shared__ int s_stop;
-  __shared__ long long s_warp[kSeqThreads / 32];
-  __shared__ long long s_base;
-  if (tid == 0) {
-    s_sum = 0.0f;
-    s_next = 0;
-  }
-  __syncthreads();
-  constexpr int CH = kSeqThreads * kSeqPer;
-  while (true) {
-    const int64_t i0 = s_next;
-    const float s = s_sum;
-    if (i0 >= N) break;
+  __shared__ float s_sum;
+  if (mean != mean) return;  // so is this sum; or the paths kernel priced nothing (bad bridge)
+  float s = 0.0f;
+  int64_t b = 0;
+  while (b < blocks) {
     const uint32_t sb = __float_as_uint(s);
-    const int se = (int)((sb >> 23) & 0xffu);
-    if (se == 0 || se == 0xff || (sb >> 31)) {  // zero, tiny or irregular running sum: one step
+    const bool zero = sb == 0u;                                      // only blocks of zeros have a pair
+    const bool normal = (sb >> 23) - 1u < 0xfeu;                      // positive and normal
+    const int e = normal ? (int)(sb >> 23) - 127 : 0;
+    int done = 0;  // blocks composed
+    if (zero || normal) {
+      const uint32_t S0 = zero ? 0u : (sb & 0x7fffffu) | 0x800000u;  // s / u
+      // the pairs of blocks b + kSeqPer * tid ..; where the prediction missed
+      // the exponent (other: this far) a warp makes the pair from the payoffs
+      SeqPair f[kSeqPer];
+      bool known = true;
+#pragma unroll
+      for (int q = 0; q < kSeqPer; q++) {
+        const int64_t bb = b + (int64_t)tid * kSeqPer + q;
+        f[q] = {kSeqNone, kSeqNone};
+        if (bb < blocks) {
+          int lo, hi;
+          seq_exponents(mean, bb, lo, hi);
+          const bool made = normal && e >= lo && e <= hi;
+          const SeqPair g = mp[(made ? e - lo : 0) * blocks + bb];
+          if (g.a1 == kSeqZeros) f[q] = {0u, 0u};
+          else if (made) f[q] = g;
+          else if (normal) known = false;
+        }
+      }
+      if (tid == 0) s_stop = kSeqThreads * kSeqPer;
+      // the first blocks unknown: made here, one per warp
+      const bool miss = __syncthreads_or(tid * kSeqPer < NW && !known);
+      if (miss) {
+        const int64_t bb = b + warp;
+        SeqPair a{kSeqNone, kSeqNone};
+        if (bb < blocks) {
+          const int n = (int)min((int64_t)kSeqBlock, N - bb * kSeqBlock);
+          float v[kSeqBlock / 32];
+          const bool zeros = seq_load_block(p, num_models, bb, n, v);
+          a = zeros ? SeqPair{0u, 0u} : seq_block_pair(v, n, e);
+        }
+        if (lane == 0) s_warp[warp] = a;
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kSeqPer; q++)
+          f[q] = tid * kSeqPer + q < NW ? s_warp[tid * kSeqPer + q] : SeqPair{kSeqNone, kSeqNone};
+        __syncthreads();
+      }
+      SeqPair mine = f[0];
+#pragma unroll
+      for (int q = 1; q < kSeqPer; q++) mine = seq_then(mine, f[q]);
+      SeqPair x = mine;  // inclusive scan over the warp
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const SeqPair y{__shfl_up_sync(0xffffffffu, x.a0, o), __shfl_up_sync(0xffffffffu, x.a1, o)};
+        if (lane >= o) x = seq_then(y, x);
+      }
+      if (lane == 31) s_warp[warp] = x;
+      SeqPair before{__shfl_up_sync(0xffffffffu, x.a0, 1), __shfl_up_sync(0xffffffffu, x.a1, 1)};
+      if (lane == 0) before = {0u, 0u};
+      __syncthreads();
+      if (warp == 0) {
+        SeqPair y = s_warp[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const SeqPair g{__shfl_up_sync(0xffffffffu, y.a0, o), __shfl_up_sync(0xffffffffu, y.a1, o)};
+          if (lane >= o) y = seq_then(g, y);
+        }
+        s_warp[lane] = y;
+      }
+      __syncthreads();
+      if (warp > 0) before = seq_then(s_warp[warp - 1], before);
+      uint32_t run = S0 + ((S0 & 1u) ? before.a1 : before.a0);  // s / u before this thread's blocks
+      const uint32_t start = run;
+      int cross = kSeqThreads * kSeqPer;
+#pragma unroll
+      for (int q = 0; q < kSeqPer; q++) {
+        const uint32_t nx = run + ((run & 1u) ? f[q].a1 : f[q].a0);
+        if (cross == kSeqThreads * kSeqPer) {
+          if (nx >= kSeqLim) cross = tid * kSeqPer + q; else run = nx;
+        }
+      }
+      if (cross < kSeqThreads * kSeqPer) atomicMin(&s_stop, cross);
+      __syncthreads();
+      done = s_stop;
+      // s / u there, from the thread whose blocks hold the stop (or the last one)
+      const int owner = min(done / kSeqPer, kSeqThreads - 1);
+      if (tid == owner) s_base = done == owner * kSeqPer ? start : run;
+      __syncthreads();
+      if (!zero) s = ldexpf((float)s_base, e - 23);  // exact: s_base < 2^24
+      b += done;
+    }
+    if (b < blocks && done < kSeqThreads * kSeqPer) {  // block b, payoff by payoff
+      const int n = (int)min((int64_t)kSeqBlock, N - b * kSeqBlock);
+      __syncthreads();
+      for (int k = tid; k < kSeqBlock; k += kSeqThreads) s_pay[k] = k < n ? p[(b * kSeqBlock + k) * num_models] : 0.0f;
       __syncthreads();
       if (tid == 0) {
-        s_sum = s + p[i0 * num_models];
-        s_next = i0 + 1;
+        float v = s;
+        if (n == kSeqBlock) {
+#pragma unroll 8
+          for (int k = 0; k < kSeqBlock; k += 4) {
+            const float4 q = *reinterpret_cast<const float4*>(s_pay + k);
+            v = (((v + q.x) + q.y) + q.z) + q.w;
+          }
+        } else {
+          for (int k = 0; k < n; k++) v = v + s_pay[k];
+        }
+        s_sum = v;
       }
       __syncthreads();
-      continue;
+      s = s_sum;
+      b++;
     }
-    const int e = se - 127;
-    const int64_t S0 = (int64_t)((sb & 0x7fffffu) | 0x800000u);  // s / u
-    const int64_t len = min((int64_t)CH, N - i0);
-    // pass 1: the first payoff of the chunk that needs a step of its own
-    if (tid == 0) s_stop = (int)len;
-    __syncthreads();
-    uint32_t t[kSeqPer];
-    int my_stop = (int)len;
-#pragma unroll
-    for (int j = 0; j < kSeqPer; j++) {
-      const int k = tid * kSeqPer + j;
-      t[j] = 0;
-      if (k < len && my_stop == (int)len && !seq_units(p[(i0 + k) * num_models], e, t[j])) my_stop = k;
-    }
-    if (my_stop < (int)len) atomicMin(&s_stop, my_stop);
-    __syncthreads();
-    const int stop = s_stop;
-    // pass 2: units before the stop, scanned; the first payoff that would
-    // carry the sum out of the binade is a stop too
-    int64_t mine = 0;
-#pragma unroll
-    for (int j = 0; j < kSeqPer; j++)
-      if (tid * kSeqPer + j < stop) mine += t[j];
-    const int64_t wex = warp_excl_scan(mine, lane);
-    if (lane == 31) s_warp[warp] = wex + mine;
-    __syncthreads();
-    if (warp == 0) {
-      const int64_t v = lane < kSeqThreads / 32 ? s_warp[lane] : 0;
-      const int64_t x = warp_excl_scan(v, lane);
-      if (lane < kSeqThreads / 32) s_warp[lane] = x;
-    }
-    __syncthreads();
-    int64_t run = S0 + s_warp[warp] + wex;  // s / u before this thread's first payoff
-    const int64_t lim = (int64_t)1 << 24;   // s / u reaching 2^24 leaves the binade
-    int cross = stop;
-#pragma unroll
-    for (int j = 0; j < kSeqPer; j++) {
-      const int k = tid * kSeqPer + j;
-      if (k < stop && cross == stop) {
-        if (run + t[j] >= lim) cross = k; else run += t[j];
-      }
-    }
-    if (cross < stop) atomicMin(&s_stop, cross);
-    __syncthreads();
-    const int q = s_stop;
-    // the sum before payoff q, from the thread whose range holds q (or the last)
-    const int owner = q < (int)len ? q / kSeqPer : kSeqThreads - 1;
-    if (tid == owner) {
-      int64_t r = S0 + s_warp[warp] + wex;
-#pragma unroll
-      for (int j = 0; j < kSeqPer; j++)
-        if (tid * kSeqPer + j < q) r += t[j];
-      s_base = r;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      float v = ldexpf((float)s_base, e - 23);  // exact: s_base < 2^24
-      int64_t nx = i0 + len;
-      if (q < (int)len) {
-        v = v + p[(i0 + q) * num_models];  // the step the sequential loop takes there
-        nx = i0 + q + 1;
-      }
-      s_sum = v;
-      s_next = nx;
-    }
-    __syncthreads();
   }
-  if (tid == 0) {
-    const float f64_order = out[m0 + mm];  // NaN when the paths kernel priced nothing (bad bridge)
-    out[m0 + mm] = f64_order != f64_order ? f64_order : s_sum / (float)num_mc_it;
-  }
+  if (tid == 0) out[m0 + mm] = s / (float)num_mc_it;
 }
 
 constexpr size_t kWarpSmem3 = sizeof(float) * OpWarpSmem<3>::kWords;
@@ -741,8 +855,14 @@ size_t payoff_bytes(const futhark_context* ctx, const op_args* q) {
   if (ctx->reduce_order != 1) return 0;
   return sizeof(float) * (size_t)std::max(0, q->num_mc_it) * (size_t)std::max(0, q->num_models);
 }
+// (reference order) the block pairs of one launch's models
+size_t maps_bytes(const futhark_context* ctx, const op_args* q) {
+  if (ctx->reduce_order != 1 || q->num_mc_it <= 0) return 0;
+  const size_t blocks = ((size_t)q->num_mc_it + kSeqBlock - 1) / kSeqBlock;
+  return sizeof(SeqPair) * kSeqMaps * blocks * (size_t)std::min(kOpModels, std::max(0, q->num_models));
+}
 size_t scratch_for(const futhark_context* ctx, const op_args* q) {
-  return partial_bytes(ctx) + dirs_bytes(q) + payoff_bytes(ctx, q) + 256;
+  return partial_bytes(ctx) + dirs_bytes(q) + maps_bytes(ctx, q) + payoff_bytes(ctx, q) + 256;
 }
 
 // Enqueues one pricing (lock held, device set, shapes valid, scratch large enough).
@@ -751,8 +871,10 @@ int op_launch(futhark_context* ctx, const op_args* q, float* out, void* scratch)
   const int c = q->contract_number;
   const bool priced = c >= 1 && c <= 3 && q->num_mc_it > 0;
   float* pay_out = priced && ctx->reduce_order == 1
-                       ? reinterpret_cast<float*>(static_cast<char*>(scratch) + partial_bytes(ctx) + dirs_bytes(q))
+                       ? reinterpret_cast<float*>(static_cast<char*>(scratch) + partial_bytes(ctx) + dirs_bytes(q) +
+                                                  maps_bytes(ctx, q))
                        : nullptr;
+  SeqPair* maps = reinterpret_cast<SeqPair*>(static_cast<char*>(scratch) + partial_bytes(ctx) + dirs_bytes(q));
   OpDev a{q->num_mc_it, q->num_bits, q->num_models, q->num_discts, q->dir_vs, q->md_cs, q->md_vols, q->md_drifts,
           q->md_sts, q->md_detvals, q->md_discts, q->bb_inds, q->bb_data, pay_out};
   double* partial = static_cast<double*>(scratch);
@@ -783,8 +905,12 @@ int op_launch(futhark_context* ctx, const op_args* q, float* out, void* scratch)
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "option pricing reduction launch");
     if (pay_out) {  // the reference's order replaces the f64 one (NaN stays NaN)
+      const int64_t blocks = ((int64_t)q->num_mc_it + kSeqBlock - 1) / kSeqBlock;
+      op_seq_maps_kernel<<<dim3((unsigned)((blocks + 7) / 8), nm), 256, 0, ctx->stream>>>(
+          pay_out, q->num_mc_it, q->num_models, m0, out, maps);
+      if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "option pricing ordered reduction launch");
       op_seq_reduce_kernel<<<nm, kSeqThreads, 0, ctx->stream>>>(pay_out, q->num_mc_it, q->num_models, m0,
-                                                                 q->num_mc_it, out);
+                                                                 q->num_mc_it, maps, out);
       e = cudaGetLastError();
       if (e != cudaSuccess) return cuda_fail(ctx, e, "option pricing ordered reduction launch");
     }

@@ -132,9 +132,10 @@ OP_API void *op_context_stream(struct futhark_context *ctx);
  * order, rounded once -- the more accurate mean.  OP_ORDER_SEQUENTIAL_F32: an
  * f32 running sum in path order, the order the reference's golden outputs
  * (the .out files of finpar/OptionPricing-data) were produced in, computed exactly; it
- * needs num_mc_it * num_models * 4 more bytes of scratch (op_scratch_bytes
- * counts them) and time for a pass over the stored payoffs.  Applies to the
- * calls that follow on this context. */
+ * needs num_mc_it * num_models * 4 more bytes of scratch and 16 per 256 paths
+ * and model (op_scratch_bytes counts them: ask it again after changing the
+ * order), and time for a pass over the stored payoffs.  Applies to the calls
+ * that follow on this context. */
 #define OP_ORDER_F64 0
 #define OP_ORDER_SEQUENTIAL_F32 1
 OP_API int op_context_set_reduction_order(struct futhark_context *ctx, int32_t order);
