@@ -47,9 +47,9 @@ __device__ __forceinline__ void dd_stencil(double xm, double x0, double xp, doub
 __global__ void __launch_bounds__(256) lvc_setup_kernel(const CalibDev* __restrict__ calibs,
                                                         double* __restrict__ tabs) {
   const CalibDev c = calibs[blockIdx.x];
-  const int X = c.numX, Y = c.numY, T = c.numT, Xp = c.Xp;
+  const int X = c.Xr, Y = c.Yr, T = c.numT, Xp = c.Xp;
   const bool line = c.kind == kKindLine;
-  const TabLayout L = tab_layout(X, Y, T, Xp, c.kind);
+  const TabLayout L = tab_layout(c.numX, c.numY, T, Xp, c.kind);
   double* tab = tabs + c.tab;
   const int tid = threadIdx.x, nt = blockDim.x;
 
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(256) lvc_setup_kernel(const CalibDev* __restri
 
   // Column tables: eX_i and 0.5 * Dxx_i[k]  (updateParams :63, explicitMethod :138-144)
   for (int i = tid; i < Xp; i += nt) {
-    double e = 0.0, h0 = 0.0, h1 = 0.0, h2 = 0.0, xv = 0.0;
+    double e = 0.0, h0 = 0.0, h1 = 0.0, h2 = 0.0, xv = i < c.numX ? kNoSpot : 0.0;
     if (i < X) {
       xv = grid_pt(i, dx, xidx, c.s0);
       e = exp(__dmul_rn(2.0, __dmul_rn(c.beta, log(xv))));
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(256) lvc_setup_kernel(const CalibDev* __restri
     }
   }
   // Row tables: 0.5 * nu^2 * Dyy_j[k]
-  for (int j = tid; j < Y; j += nt) {
+  for (int j = tid; j < c.numY; j += nt) {
     double g0 = 0.0, g1 = 0.0, g2 = 0.0;
     if (j > 0 && j < Y - 1) {
       double d0, d1, d2;
@@ -163,7 +163,7 @@ __device__ __forceinline__ int find_calib(const int64_t* __restrict__ start, int
 // co: [kLineK][4] shared memory of this warp.
 __device__ __forceinline__ void y_pivots(const CalibDev& c, int k0, double* __restrict__ tabs, double (*co)[4]) {
   const int lane = threadIdx.x & 31;
-  const int Y = c.numY, steps = c.numT - 1;
+  const int Y = c.numY, steps = c.numT - 1;  // a padding row's coefficients are zero: b' = dt, no multipliers
   const bool line = c.kind == kKindLine;
   const TabLayout L = tab_layout(c.numX, Y, c.numT, c.Xp, c.kind);
   double* tab = tabs + c.tab;
@@ -185,7 +185,7 @@ __device__ __forceinline__ void y_pivots(const CalibDev& c, int k0, double* __re
       co[lane][0] = a * cprev;
       co[lane][1] = 0.5 * rc[1];
       co[lane][2] = a;
-      co[lane][3] = j == Y - 1 ? 0.0 : cc;
+      co[lane][3] = j == c.Yr - 1 ? 0.0 : cc;
     }
     __syncwarp();
     if (n == kLineK) {
@@ -257,9 +257,9 @@ template <typename PV>
 __device__ __forceinline__ void x_pivots(const CalibDev& c, int64_t r0, double* __restrict__ tabs,
                                          PV* __restrict__ piv, double (*co)[4], double (*tile)[kPivotCols + 1]) {
   const int lane = threadIdx.x & 31;
-  const int X = c.numX, Y = c.numY;
+  const int X = c.Xr, Y = c.numY;
   const bool line = c.kind == kKindLine;
-  const TabLayout L = tab_layout(X, Y, c.numT, c.Xp, c.kind);
+  const TabLayout L = tab_layout(c.numX, Y, c.numT, c.Xp, c.kind);
   double* tab = tabs + c.tab;
   const int64_t rows = (int64_t)(c.numT - 1) * Y;
   const int nr = (int)min((int64_t)32, rows - r0);  // rows of this group
@@ -289,9 +289,11 @@ __device__ __forceinline__ void x_pivots(const CalibDev& c, int64_t r0, double* 
   fetch(lane);
   // e_j of the step: exp(2 (y_j - 0.5 nu^2 t_k))  (updateParams, :63)
   const double tn = __ddiv_rn(__dmul_rn(c.t, (double)k), __dsub_rn((double)c.numT, 1.0));
-  const double dy = __ddiv_rn(__dmul_rn(__dmul_rn(10.0, c.nu), sqrt(c.t)), (double)Y);
+  const double dy = __ddiv_rn(__dmul_rn(__dmul_rn(10.0, c.nu), sqrt(c.t)), (double)c.Yr);
   const double yj = grid_pt(j, dy, (double)c.yindex, log(c.alpha));
-  const double e = exp(__dmul_rn(2.0, __dsub_rn(yj, __dmul_rn(__dmul_rn(__dmul_rn(0.5, c.nu), c.nu), tn))));
+  const double e = j < c.Yr
+                       ? exp(__dmul_rn(2.0, __dsub_rn(yj, __dmul_rn(__dmul_rn(__dmul_rn(0.5, c.nu), c.nu), tn))))
+                       : 0.0;
   if (lane < nr) tab[line ? L.stab + ((int64_t)k * Y + j) * 8 + kSlotE : L.eyt + (int64_t)k * L.eyt_ld + j] = e;
   double rb = 0.0, c_prev = 0.0;  // 1/b' and c of the column before: zero before the first
   for (int c0 = 0; c0 < LD; c0 += kPivotCols) {

@@ -30,10 +30,19 @@ enum : int32_t {
 };
 
 // One calibration, as the device sees it.  Filled by the host runtime.
+//
+// numX and numY are those of the tables and the on-chip grid.  The paired kernel
+// runs whole tiles, so for it they are the calibration's own sizes Xr, Yr rounded
+// up; for the other kernels they are Xr, Yr.  What padding adds is uncoupled from
+// the grid: columns and rows of zero coefficients, columns whose payoff is zero
+// (their spot is kNoSpot).  Xp is numX, or for the chunk family numX padded to a
+// power of two >= 8.
+constexpr double kNoSpot = -1e300;
 struct CalibDev {
-  int32_t numX, numY, numT, Xp;      // Xp: numX padded to a power of two >= 8
+  int32_t numX, numY, numT, Xp;      // grid and tables (below); Xp: columns of the column tables
   int32_t outer, xindex, yindex, C;  // C: CTAs (cluster size) per instance
-  int32_t kind, Ycs, ld, pad1;       // kernel family; rows per CTA; line family: row stride
+  int32_t kind, Ycs, ld;             // kernel family; rows per CTA; line family: row stride
+  int16_t Xr, Yr;                    // the calibration's own numX, numY
   double s0, t, alpha, nu, beta;
   int64_t tab;  // offset (doubles) of the operator tables in the table arena
   int64_t piv;  // offset (elements) of the X-direction pivots in the pivot arena

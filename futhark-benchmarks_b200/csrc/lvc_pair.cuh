@@ -15,8 +15,11 @@
 // reading one 16-byte pair from 32 consecutive rows fall into 4 conflict-free
 // wavefronts (8 lanes cover the 32 banks), and rows start 16-byte aligned for
 // the pair accesses of the Y sweep.  Columns numX and numX + 1 are zero.
-// Needs numX % (32 * UPW) == 0 (whole Y units), rows per CTA % 32 == 0 and
-// numY = cluster size x rows per CTA.
+// The on-chip grid is made of whole tiles, columns a multiple of 32 * UPW (whole
+// Y units) and rows per CTA a multiple of 32; a grid of other sizes is padded
+// (CalibDev).  Padding 101 x 75 to 128 x 96 is 1.6 times the cells, at four times
+// the rate of the kernel for any sizes (50 strikes, 129 steps: 2078 us there, 760
+// here).
 //
 // UPW (units per warp) = 2: each warp owns two X units (two independent
 // recurrence chains per lane) and one 64-column Y unit (two columns per lane);
@@ -218,7 +221,7 @@ __global__ void __launch_bounds__(NT, (PairMinBlocks<S, NT, UPW>::v)) lvc_line_p
     // cluster -- every rank has read the last block maps this CTA pushed to it.
     if (clustered) cg::this_cluster().sync(); else __syncthreads();
     // setPayoff (:46-47) on the block and the halo rows (zero at the global
-    // boundary and in the two padding columns)
+    // boundary and in the two columns beyond X)
     for (int e = tid; e < (Ycs + 2) * LD; e += NT) {
       const int r = e / LD, i = e - r * LD;
       const bool boundary = (r == 0 && rank == 0) || (r == Ycs + 1 && rank == C - 1);

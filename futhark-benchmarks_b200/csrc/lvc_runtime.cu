@@ -311,6 +311,8 @@ struct lvc_plan {
   double rollback_ms = 0.0;
   DevicePool* pool = nullptr;  // where the buffers come from (null: cudaMalloc)
   bool use_graph = true;       // capture one run into a CUDA graph
+  bool pad = true;             // built-in shapes may pad the grid
+  bool alone = false;          // an entry point's call: the shape may go by the number of strikes
   int max_sms = 0;             // cap on the SMs a launch may occupy (0: all, <0: one CTA per item)
   double sms = 0.0;            // SMs the widest launch occupies
   int n_streams = 1;           // streams the launch classes fork over
@@ -417,13 +419,16 @@ RbFn<S, PV> rollback_fn(int kind, int NT, int KX, bool gs, bool full = false, bo
   if (kind == kKindLine && pair && upw == 1) {
     if (NT == 64) return lvc_line_pair_kernel<S, PV, 64, 1>;
     if (NT == 128) return lvc_line_pair_kernel<S, PV, 128, 1>;
+    if (NT == 192) return lvc_line_pair_kernel<S, PV, 192, 1>;
     if (NT == 256) return lvc_line_pair_kernel<S, PV, 256, 1>;
+    if (NT == 384) return lvc_line_pair_kernel<S, PV, 384, 1>;
     if (NT == 512) return lvc_line_pair_kernel<S, PV, 512, 1>;
     return nullptr;
   }
   if (kind == kKindLine && pair) {
     if (NT == 64) return lvc_line_pair_kernel<S, PV, 64, 2>;
     if (NT == 128) return lvc_line_pair_kernel<S, PV, 128, 2>;
+    if (NT == 192) return lvc_line_pair_kernel<S, PV, 192, 2>;
     if (NT == 256) return lvc_line_pair_kernel<S, PV, 256, 2>;
     return nullptr;
   }
@@ -485,23 +490,27 @@ bool line_full_cfg(int X, int Y, int C, int max_smem, Config& cf) {
   return true;
 }
 
-// Paired line kernel on full tiles: upw = 2 (two X units and one 64-column
-// Y unit per warp, numX % 64 == 0) or upw = 1 (one X unit and one 32-column
-// Y unit per warp, twice the warps).
+// Paired line kernel: upw = 2 (two X units and one 64-column Y unit per warp)
+// or upw = 1 (one X unit and one 32-column Y unit per warp, twice the warps),
+// the grid padded to whole tiles -- columns to a multiple of 32 * upw, rows to C
+// CTAs of the least multiple of 32.
 template <typename S>
 bool line_pair_cfg(int X, int Y, int C, int max_smem, Config& cf, int upw = 2) {
-  if (X > 256 || X % (32 * upw) || Y % C || (Y / C) % 32) return false;
-  const int Ycs = Y / C;
-  const int units = X * Ycs / 512;  // X units of 32 rows x 16 columns
+  const int tile = 32 * upw;
+  const int Xt = ceil_div(X, tile) * tile;
+  const int Ycs = ceil_div(ceil_div(Y, C), 32) * 32;
+  if (Xt > 256 || (C - 1) * Ycs >= Y) return false;  // a CTA would own no row
+  const int units = Xt * Ycs / 512;  // X units of 32 rows x 16 columns
   const int NW = units / upw;
-  if (NW * upw != units || NW < 2 || NW > (upw == 2 ? 8 : 16) || (NW & (NW - 1))) return false;
-  const PairLayout F = pair_layout<S>(X, Ycs, upw, C);
+  const bool built = NW == 2 || NW == 4 || NW == 6 || NW == 8 || (upw == 1 && (NW == 12 || NW == 16));
+  if (NW * upw != units || !built) return false;
+  const PairLayout F = pair_layout<S>(Xt, Ycs, upw, C);
   if (F.Ux != units || F.Uy != NW || F.total > max_smem) return false;
   cf.kind = kKindLine;
   cf.full = false;
   cf.pair = true;
   cf.upw = upw;
-  cf.ld = pair_ld(X);
+  cf.ld = pair_ld(Xt);
   cf.NT = 32 * NW;
   cf.KX = kLineK;
   cf.C = C;
@@ -510,6 +519,17 @@ bool line_pair_cfg(int X, int Y, int C, int max_smem, Config& cf, int upw = 2) {
   cf.smem_bytes = (size_t)F.total;
   cf.grid_elems = 0;
   return true;
+}
+
+// Columns and rows of a configuration's tables, and the column tables' width.
+int tab_cols(const Config& cf, int X) { return cf.pair ? cf.ld - 2 : X; }
+int tab_rows(const Config& cf, int Y) { return cf.pair ? cf.C * cf.Ycs : Y; }
+int tab_xp(const Config& cf, int X) { return cf.pair ? tab_cols(cf, X) : std::max(8, pow2ceil(X)); }
+int64_t tab_count(const Config& cf, int X, int Y, int T) {
+  return al2(tab_layout(tab_cols(cf, X), tab_rows(cf, Y), T, tab_xp(cf, X), cf.kind).total);
+}
+int64_t piv_count(const Config& cf, int X, int Y, int T) {
+  return (piv_elems(X, tab_rows(cf, Y), T, tab_xp(cf, X), cf.kind, cf.ld) + 3) & ~int64_t(3);
 }
 
 // Line family, any sizes: one lane per grid line; needs numX <= 256 and at
@@ -564,16 +584,23 @@ bool chunk_cfg(int X, int Y, int C, int max_smem, bool gstate, Config& cf) {
   return true;
 }
 
-// Built-in choice: the smallest cluster the line family fits in (paired
-// kernel with two units per warp, then with one unit per warp -- numX == 32
-// --, then full tiles, then any sizes), else the chunk family on chip, else
-// the chunk family on HBM.
+// A grid of whole tiles in power-of-two splits: the sizes the paired kernel runs
+// without padding.
+bool whole_tiles(int X, int Y) {
+  auto pow2 = [](int v) { return (v & (v - 1)) == 0; };
+  return X % 32 == 0 && Y % 32 == 0 && pow2(X) && pow2(Y);
+}
+
+// The smallest cluster the line family fits in (paired kernel on whole tiles
+// with two units per warp, then with one unit per warp -- numX == 32 --, then
+// full tiles, then any sizes), else the chunk family on chip, else the chunk
+// family on HBM.
 template <typename S>
-Config default_config(int X, int Y, int max_smem) {
+Config unpadded_config(int X, int Y, int max_smem) {
   Config cf;
   for (int C = 1; C <= kMaxCluster; C *= 2) {
-    if (line_pair_cfg<S>(X, Y, C, max_smem, cf)) return cf;
-    if (line_pair_cfg<S>(X, Y, C, max_smem, cf, 1)) return cf;  // numX == 32
+    if (whole_tiles(X, Y) && line_pair_cfg<S>(X, Y, C, max_smem, cf) && tab_cols(cf, X) == X) return cf;
+    if (whole_tiles(X, Y) && line_pair_cfg<S>(X, Y, C, max_smem, cf, 1)) return cf;
     if (line_full_cfg<S>(X, Y, C, max_smem, cf)) return cf;
     if (line_generic_cfg<S>(X, Y, C, max_smem, cf)) return cf;
   }
@@ -581,6 +608,74 @@ Config default_config(int X, int Y, int max_smem) {
     if (chunk_cfg<S>(X, Y, C, max_smem, false, cf)) return cf;
   chunk_cfg<S>(X, Y, 1, max_smem, true, cf);
   return cf;
+}
+
+// The paired kernel's splits of a grid into CTAs of the least rows: 1, 2, 4, ..
+// for a grid of whole tiles, 1 .. 8 (a portable cluster) for one to be padded.
+template <typename S>
+std::vector<Config> pair_configs(int X, int Y, int max_smem) {
+  std::vector<Config> v;
+  Config cf;
+  const bool tiles = whole_tiles(X, Y);
+  for (int C = 1; C <= (tiles ? kMaxCluster : 8); C += tiles ? C : 1)
+    for (int upw = 2; upw >= 1; upw--)
+      if (line_pair_cfg<S>(X, Y, C, max_smem, cf, upw) && (!tiles || tab_cols(cf, X) == X)) v.push_back(cf);
+  return v;
+}
+
+// What a time step of the paired kernel costs under a configuration, in
+// microseconds: the chip's throughput at `outer` strikes (0: many, and the
+// cost is relative), or a step's latency where the strikes do not fill it.
+// From measurements on 43 grid sizes from 3 x 3 to 256 x 256 at 8, 64 and 400
+// strikes, f64: per 1000 cells and strike 5.2 ns unclustered; 6.2 ns in clusters
+// of CTAs of at most 4096 cells, two of which share an SM, so that one computes
+// while the other exchanges, and 6.9 above (128 x 128 in four CTAs 39.3 against
+// 41.9 us a step at 400 strikes, 128 x 256 in eight 82.9 against 93.2); a unit
+// per warp in clusters 7.8; six warps, which leave two schedulers one warp each,
+// 8.3.  A step alone: 2.6, 2.9, 3.7, 5.7 us for a CTA of 1024 .. 8192 cells, and
+// the exchanges make that 4.5, 4.9, 5.4, 7.3 in a cluster.  With f32 state two
+// CTAs of the two-unit kernel share an SM at any size, and a unit per warp costs
+// 1.8 times as much.
+template <typename S>
+double pair_cost(const Config& cf, int X, int Y, int outer) {
+  const double cta = (double)tab_cols(cf, X) * cf.Ycs, cells = cta * cf.C;
+  const bool f64 = sizeof(S) == 8, clustered = cf.C > 1;
+  double per = clustered ? 6.2e-6 : 5.2e-6;
+  if (f64 && clustered && cta > 4096) per *= 1.12;
+  if (f64 && clustered && cf.upw == 2 && cf.NT == 192) per *= 1.2;
+  if (cf.upw == 1) per *= !f64 ? 1.8 : clustered ? 1.25 : 1.08;
+  const double chip = per * cells;
+  if (outer <= 0) return chip;
+  const double alone = clustered ? 4.3 + 0.34e-3 * cta : 2.1 + 0.43e-3 * cta;
+  // whichever is longer; the other one decides between near equals
+  return std::max(outer * chip, alone) + 0.05 * std::min(outer * chip, alone);
+}
+
+// Built-in choice: the paired kernel's cheapest split, where there is one (numX
+// up to 256 on chip).  Padding a grid to whole tiles costs up to four times its
+// cells and still beats the kernels for any sizes on all but the thinnest grids:
+// 101 x 75 at 400 strikes 31 us a step against 83, 240 x 240 201 against 494,
+// 50 x 50 8.4 against 21; 3 x 3 3.1 against 3.2, 200 x 7 16.5 against 15.3.
+// outer: the strikes of a call that runs alone (the entry points), 0 for batches
+// and serving, where the shape -- and with it the last bits of a price -- may not
+// depend on what a calibration is batched with.  There whole tiles keep the
+// smallest cluster: among other launch classes two small CTAs per SM are worth
+// less than they are alone (the 512-calibration mix takes 254.5 ms with 128 x 128,
+// 128 x 256 and 64 x 256 in the smallest clusters and 267 in ones of CTAs of 4096
+// cells).
+template <typename S>
+Config default_config(int X, int Y, int max_smem, int outer = 0) {
+  if (outer <= 0 && whole_tiles(X, Y)) return unpadded_config<S>(X, Y, max_smem);
+  Config best;
+  double best_cost = 0.0;
+  for (const Config& cf : pair_configs<S>(X, Y, max_smem)) {
+    const double cost = pair_cost<S>(cf, X, Y, outer);
+    if (best_cost == 0.0 || cost < best_cost) {
+      best = cf;
+      best_cost = cost;
+    }
+  }
+  return best_cost > 0.0 ? best : unpadded_config<S>(X, Y, max_smem);
 }
 
 // Every configuration that can run an X x Y grid: the search space of the
@@ -591,9 +686,8 @@ template <typename S>
 std::vector<Config> enum_configs(int X, int Y, int max_smem) {
   std::vector<Config> v;
   Config cf;
+  v = pair_configs<S>(X, Y, max_smem);
   for (int C = 1; C <= kMaxCluster; C *= 2) {
-    if (line_pair_cfg<S>(X, Y, C, max_smem, cf)) v.push_back(cf);
-    if (line_pair_cfg<S>(X, Y, C, max_smem, cf, 1)) v.push_back(cf);
     if (line_full_cfg<S>(X, Y, C, max_smem, cf)) v.push_back(cf);
     if (line_generic_cfg<S>(X, Y, C, max_smem, cf) && (C == 1 || cf.Ycs >= 16)) v.push_back(cf);
   }
@@ -620,12 +714,12 @@ template <typename S>
 int precision_of() { return sizeof(S) == sizeof(double) ? LVC_F64 : LVC_F32_STATE; }
 
 // The configuration of an X x Y grid: the context's tuned shape, else the
-// built-in choice.
+// built-in choice (pad == false: without padding, for a caller short of memory).
 template <typename S>
-Config choose_config(const futhark_context* ctx, int X, int Y) {
+Config choose_config(const futhark_context* ctx, int X, int Y, bool pad = true, int outer = 0) {
   auto it = ctx->shapes.find(TuneKey{X, Y, precision_of<S>()});
   if (it != ctx->shapes.end()) return it->second.cf;
-  return default_config<S>(X, Y, ctx->max_smem);
+  return pad ? default_config<S>(X, Y, ctx->max_smem, outer) : unpadded_config<S>(X, Y, ctx->max_smem);
 }
 
 template <typename S, typename PV>
@@ -802,28 +896,29 @@ int plan_build(futhark_context* ctx, const lvc_calibration* cs, int n, lvc_plan*
   for (int i = 0; i < n; i++) {
     const lvc_calibration& c = cs[i];
     if (int rc = validate(ctx, c, i)) return rc;
-    const Config cf = choose_config<S>(ctx, c.numX, c.numY);
+    const Config cf = choose_config<S>(ctx, c.numX, c.numY, P->pad, P->alone ? c.outer : 0);
     P->cfgs[i] = cf;
     CalibDev& d = P->calibs[i];
-    d.numX = c.numX;
-    d.numY = c.numY;
+    d.numX = tab_cols(cf, c.numX);
+    d.numY = tab_rows(cf, c.numY);
     d.numT = c.numT;
-    d.Xp = std::max(8, pow2ceil(c.numX));
+    d.Xp = tab_xp(cf, c.numX);
     d.outer = c.outer;
     d.C = cf.C;
     d.kind = cf.kind;
     d.Ycs = cf.Ycs;
     d.ld = cf.ld;
-    d.pad1 = 0;
+    d.Xr = (int16_t)c.numX;
+    d.Yr = (int16_t)c.numY;
     fill_scalars(d, c);
     d.tab = tab_off;
-    tab_off += al2(tab_layout(c.numX, c.numY, c.numT, d.Xp, d.kind).total);
+    tab_off += tab_count(cf, c.numX, c.numY, c.numT);
     d.piv = piv_off;
-    piv_off += (piv_elems(c.numX, c.numY, c.numT, d.Xp, d.kind, d.ld) + 3) & ~int64_t(3);
+    piv_off += piv_count(cf, c.numX, c.numY, c.numT);
     d.out = out_off;
     out_off += c.outer;
     yg_start[i + 1] = yg_start[i] + y_groups(c.numT);
-    xg_start[i + 1] = xg_start[i] + x_groups(c.numY, c.numT);
+    xg_start[i + 1] = xg_start[i] + x_groups(d.numY, c.numT);
     const auto key = std::make_tuple(cf.kind, cf.NT, cf.KX, cf.C, cf.gstate, cf.full, cf.pair, cf.upw);
     auto& cls = classes[key];
     auto it = class_cfg.find(key);
@@ -939,7 +1034,7 @@ int plan_build(futhark_context* ctx, const lvc_calibration* cs, int n, lvc_plan*
 
 int plan_new_locked(futhark_context* ctx, const lvc_calibration* cs, int n, int precision,
                     lvc_plan** out, DevicePool* pool = nullptr, bool use_graph = true,
-                    int max_sms = 0) {
+                    int max_sms = 0, bool pad = true, bool alone = false) {
   if (!ctx->ok) return set_error(ctx, FUTHARK_PROGRAM_ERROR, "context has no usable CUDA device");
   if (n < 0 || (n > 0 && !cs)) return set_error(ctx, FUTHARK_PROGRAM_ERROR, "bad calibration list");
   if (precision != LVC_F64 && precision != LVC_F32_STATE)
@@ -950,6 +1045,8 @@ int plan_new_locked(futhark_context* ctx, const lvc_calibration* cs, int n, int 
   P->pool = pool;
   P->use_graph = use_graph;
   P->max_sms = max_sms;
+  P->pad = pad;
+  P->alone = alone;
   P->shapes_gen = ctx->shapes_gen;
   if (use_graph && max_sms == 0) {  // batch plans follow the context's tuning
     P->max_sms = grid_mode(ctx->tuning, precision) == 1 ? -1 : 0;
@@ -1029,7 +1126,9 @@ int entry_run(futhark_context* ctx, const lvc_calibration& c) {
   }
   if (!P) {
     if (!ctx->pool) ctx->pool = new DevicePool();
-    if (int rc = plan_new_locked(ctx, &c, 1, LVC_F64, &P, ctx->pool, /*use_graph=*/false)) return rc;
+    if (int rc = plan_new_locked(ctx, &c, 1, LVC_F64, &P, ctx->pool, /*use_graph=*/false, /*max_sms=*/0, /*pad=*/true,
+                                 /*alone=*/true))
+      return rc;
     ctx->entry_plan = P;
   } else if (int rc = set_params_locked(ctx, P, &c, 1)) {
     return rc;
@@ -1944,9 +2043,8 @@ struct NoallocCarve {
   size_t o_calib, o_err, o_starts, o_items, o_tabs, o_piv, need;
 };
 NoallocCarve noalloc_carve(const Config& cf, int outer, int numX, int numY, int numT) {
-  const int Xp = std::max(8, pow2ceil(numX));
-  const int64_t tab_elems = al2(tab_layout(numX, numY, numT, Xp, cf.kind).total);
-  const int64_t piv_n = (piv_elems(numX, numY, numT, Xp, cf.kind, cf.ld) + 3) & ~int64_t(3);
+  const int64_t tab_elems = tab_count(cf, numX, numY, numT);
+  const int64_t piv_n = piv_count(cf, numX, numY, numT);
   NoallocCarve c;
   c.o_calib = 0;
   c.o_err = up256(c.o_calib + sizeof(CalibDev));
@@ -1958,12 +2056,23 @@ NoallocCarve noalloc_carve(const Config& cf, int outer, int numX, int numY, int 
   return c;
 }
 
+// The shape the no-allocation entry point runs: the context's choice, or, when
+// its padded tables do not fit the static scratch and nothing is pinned, the
+// shape without padding.
+Config noalloc_config(const futhark_context* ctx, int outer, int numX, int numY, int numT) {
+  const Config cf = choose_config<double>(ctx, numX, numY, /*pad=*/true, outer);
+  if (!cf.pair || noalloc_carve(cf, outer, numX, numY, numT).need <= kNoAllocScratchBytes ||
+      ctx->shapes.count(TuneKey{numX, numY, LVC_F64}))
+    return cf;
+  return unpadded_config<double>(numX, numY, ctx->max_smem);
+}
+
 extern "C" int64_t lvc_entry_main_f64_noalloc_bytes(struct futhark_context* ctx, const int32_t outer,
                                                     const int32_t numX, const int32_t numY, const int32_t numT) {
   if (!ctx) return -1;
   std::lock_guard<std::mutex> g(ctx->mu);
   if (outer < 0 || numX < 3 || numY < 3 || numT < 1 || numX > kMaxNumX || numY > kMaxNumY) return -1;
-  const Config cf = choose_config<double>(ctx, numX, numY);
+  const Config cf = noalloc_config(ctx, outer, numX, numY, numT);
   if (cf.gstate) return -1;
   return (int64_t)noalloc_carve(cf, outer, numX, numY, numT).need;
 }
@@ -1982,22 +2091,24 @@ extern "C" int lvc_entry_main_f64_noalloc(struct futhark_context* ctx, double* p
   unsigned char* base = nullptr;
   if (int rc = noalloc_scratch(ctx, &base)) return rc;
 
-  const Config cf = choose_config<double>(ctx, numX, numY);
+  const Config cf = noalloc_config(ctx, outer, numX, numY, numT);
   if (cf.gstate)
     return set_error(ctx, FUTHARK_PROGRAM_ERROR,
                      "lvc_entry_main_f64_noalloc: this grid does not fit on chip; its HBM state "
                      "needs the allocating entry point futhark_entry_main_f64");
   CalibDev d;
   memset(&d, 0, sizeof d);
-  d.numX = numX;
-  d.numY = numY;
+  d.numX = tab_cols(cf, numX);
+  d.numY = tab_rows(cf, numY);
   d.numT = numT;
-  d.Xp = std::max(8, pow2ceil(numX));
+  d.Xp = tab_xp(cf, numX);
   d.outer = outer;
   d.C = cf.C;
   d.kind = cf.kind;
   d.Ycs = cf.Ycs;
   d.ld = cf.ld;
+  d.Xr = (int16_t)numX;
+  d.Yr = (int16_t)numY;
   fill_scalars(d, c);
   d.tab = 0;
   d.piv = 0;
@@ -2019,7 +2130,7 @@ extern "C" int lvc_entry_main_f64_noalloc(struct futhark_context* ctx, double* p
   Item* d_items = reinterpret_cast<Item*>(base + o_items);
   double* d_tabs = reinterpret_cast<double*>(base + o_tabs);
   double* d_piv = reinterpret_cast<double*>(base + o_piv);
-  const int64_t starts[4] = {0, y_groups(numT), 0, x_groups(numY, numT)};
+  const int64_t starts[4] = {0, y_groups(numT), 0, x_groups(d.numY, numT)};
   cudaStream_t s = ctx->stream;
 
   // the array keeps the previous call's contents: reset what must start at zero
@@ -2220,14 +2331,13 @@ void server_retire(lvc_server* S) {
 
 // Device bytes a one-calibration plan takes (tables, pivots, work list,
 // prices, state scratch), from the same layouts the plan builder uses.
-size_t request_bytes(const futhark_context* ctx, const lvc_calibration& c, int precision) {
+size_t request_bytes(const futhark_context* ctx, const lvc_calibration& c, int precision, bool pad = true) {
   const bool f64 = precision == LVC_F64;
-  const Config cf = f64 ? choose_config<double>(ctx, c.numX, c.numY)
-                        : choose_config<float>(ctx, c.numX, c.numY);
-  const int Xp = std::max(8, pow2ceil(c.numX));
+  const Config cf = f64 ? choose_config<double>(ctx, c.numX, c.numY, pad)
+                        : choose_config<float>(ctx, c.numX, c.numY, pad);
   const size_t ps = f64 ? 8 : 4;
-  size_t b = 8 * (size_t)al2(tab_layout(c.numX, c.numY, c.numT, Xp, cf.kind).total);
-  b += ps * (size_t)(piv_elems(c.numX, c.numY, c.numT, Xp, cf.kind, cf.ld) + 4);
+  size_t b = 8 * (size_t)tab_count(cf, c.numX, c.numY, c.numT);
+  b += ps * (size_t)(piv_count(cf, c.numX, c.numY, c.numT) + 4);
   b += 16 * (size_t)c.outer + 4096;
   if (cf.gstate) b += ps * (size_t)cf.grid_elems * 148 * 4;
   return b + 8 * 256;  // allocation rounding
@@ -2258,6 +2368,7 @@ bool server_admit(lvc_server* S, std::unique_lock<std::mutex>& lk) {
   size_t bytes = 0;
   auto free_bytes = [&]() { return S->pool.budget > S->pool.in_use ? S->pool.budget - S->pool.in_use : 0; };
   double take_work = 0, first_work = 0;
+  bool pad = true;
   while (!S->pending.empty() && (int)take.size() < S->cfg.max_batch_requests &&
          S->inflight_requests + (int)take.size() < S->cfg.max_inflight_requests) {
     auto pit = next_pick();
@@ -2265,7 +2376,13 @@ bool server_admit(lvc_server* S, std::unique_lock<std::mutex>& lk) {
     // a batch completes with its largest request: a small request joins no
     // batch of requests much larger than itself
     if (!take.empty() && r->work > kBatchSpread * first_work) break;
-    const size_t rb = request_bytes(&S->sctx, r->c, S->cfg.precision);
+    size_t rb = request_bytes(&S->sctx, r->c, S->cfg.precision);
+    // only without padding does it fit the budget: a batch of its own
+    const bool no_pad = rb > S->pool.budget;
+    if (no_pad) {
+      rb = request_bytes(&S->sctx, r->c, S->cfg.precision, /*pad=*/false);
+      if (rb <= S->pool.budget && !take.empty()) break;
+    }
     if (rb > S->pool.budget) {  // can never fit: fail it now
       S->pending.erase(pit);
       r->status = 2;
@@ -2289,6 +2406,10 @@ bool server_admit(lvc_server* S, std::unique_lock<std::mutex>& lk) {
     take_work += r->work;
     bytes += rb;
     S->pending.erase(pit);
+    if (no_pad) {
+      pad = false;
+      break;
+    }
   }
   if (take.empty()) return false;
   // a free stream: a small batch prefers the high-priority ones, a large one
@@ -2333,7 +2454,7 @@ bool server_admit(lvc_server* S, std::unique_lock<std::mutex>& lk) {
     e = cudaMemcpyAsync(P->d_calibs, P->calibs.data(), sizeof(CalibDev), cudaMemcpyHostToDevice, st);
   } else {
     rc = plan_new_locked(&S->sctx, cs.data(), (int)cs.size(), S->cfg.precision, &P, &S->pool,
-                         /*use_graph=*/false, /*max_sms=*/-1);
+                         /*use_graph=*/false, /*max_sms=*/-1, pad);
   }
   SrvBatch* b = nullptr;
   if (!rc && e == cudaSuccess) {
