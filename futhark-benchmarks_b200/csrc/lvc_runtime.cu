@@ -173,15 +173,17 @@ struct DevicePool {
     std::lock_guard<std::mutex> g(mu);
     trim_locked();
   }
+  // Neighbours merge inside a block from cudaMalloc only: a copy that spans two of
+  // them is an invalid argument, though their addresses may be adjacent.
   void insert_free(char* p, size_t sz) {
     auto nx = free_.lower_bound(p);
-    if (nx != free_.end() && p + sz == nx->first) {
+    if (nx != free_.end() && p + sz == nx->first && !blocks.count(nx->first)) {
       sz += nx->second;
       nx = free_.erase(nx);
     }
     if (nx != free_.begin()) {
       auto pv = std::prev(nx);
-      if (pv->first + pv->second == p) {
+      if (pv->first + pv->second == p && !blocks.count(p)) {
         pv->second += sz;
         return;
       }
