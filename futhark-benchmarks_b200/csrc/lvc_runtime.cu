@@ -13,7 +13,6 @@
 //     the classes forked over several streams (largest class first) so their
 //     tails overlap, captured once into a CUDA graph.
 #include <cuda_runtime.h>
-#include <cudaTypedefs.h>  // the driver's cuTensorMapEncodeTiled signature
 
 #include <algorithm>
 #include <chrono>
@@ -339,12 +338,7 @@ struct futhark_context {
   cudaStream_t aux[kMaxAux] = {};  // fork streams of the batch plans
   std::map<std::tuple<int, int, int>, TunedShape> shapes;  // (numX, numY, precision) -> tuned shape
   uint64_t shapes_gen = 0;  // bumped on every change of `shapes`
-  // tridiagonal solves: the tensor maps of the last batch that took the
-  // tensor-copy kernel, reused while its four inputs and shape repeat, and
-  // the kernels whose shared-memory limit is already raised on this device
-  const float* tri_map_src[4] = {};
-  int64_t tri_map_rows = -1, tri_map_m = -1;
-  CUtensorMap tri_maps[4];
+  // tridiagonal kernels whose shared-memory limit is already raised on this device
   std::set<const void*> tri_smem_raised;
 };
 
@@ -2759,103 +2753,63 @@ int tridag_check_locked(futhark_context* ctx) {
   return 0;
 }
 
-// Enqueues one batched solve on ctx->stream (device pointers).  Called with
-// ctx->mu held.  m <= 256: the tensor-memory kernel; m <= 400: the
-// streaming kernel, no scratch; larger m: scratch from the context's device
-// pool (stream-ordered: every user of that pool runs on ctx->stream).
-// cuTensorMapEncodeTiled from the driver, looked up once through the runtime
-// (the library does not link against the driver library itself); null where
-// the driver does not offer it.
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-  });
-  return fn;
-}
-
-// The [rows / 4][4m] group view of one input of a batch with odd m and
-// rows % 4 == 0, in boxes of kTriTmaGroups groups x kTriTmaBox floats
-// (lvc_tridag_tma_kernel); false where it cannot be made (no encoder, a base
-// address off the 16-byte grid the tensor copies need).
-bool tri_group_map(CUtensorMap* map, const float* p, int64_t rows, int64_t m) {
-  const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-  if (!enc || (reinterpret_cast<uintptr_t>(p) & 15u) != 0) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)(4 * m), (cuuint64_t)(rows / 4)};
-  const cuuint64_t strides[1] = {(cuuint64_t)(4 * m) * sizeof(float)};
-  const cuuint32_t box[2] = {(cuuint32_t)kTriTmaBox, (cuuint32_t)kTriTmaGroups};
-  const cuuint32_t estr[2] = {1, 1};
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(p), dims, strides, box, estr,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// Raises a tridiagonal kernel's dynamic shared-memory limit once per context
-// (each kernel instance always asks for the same size).
-int tri_smem_limit(futhark_context* ctx, const void* fn, size_t bytes) {
+// Raises a tridiagonal kernel's dynamic shared-memory limit to the device's once
+// per context.
+int tri_smem_limit(futhark_context* ctx, const void* fn) {
   if (ctx->tri_smem_raised.count(fn)) return 0;
-  LVC_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  LVC_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->max_smem));
   ctx->tri_smem_raised.insert(fn);
   return 0;
 }
 
+// Systems per warp of the whole-row kernel, or 0 for the kernel that reads rows in
+// place.  The batch runs in rounds of what the SMs' shared memory holds, so the
+// tile is the one with the fewest rounds, or the fewest tiles for as many.  Between
+// near equals FORM 0, bound by latency, takes more and smaller tiles, FORM 1, with
+// three times the instructions, fewer and larger ones (57600 x 115, FORM 0: 34.1 us
+// in tiles of 20, 36.6 in 12 or 28, 39.0 in 32; FORM 1: 51, 63, 50 and 56, 49 in
+// 24).  Beyond 1600 elements a tile is 8 systems or fewer, and reading in place
+// wins once there are more than about 16 rounds (20000 x 2000: 2340 us in 34
+// rounds against 2200; 500 x 2000: 71 against 1195).
+int tri_row_tile(const futhark_context* ctx, int form, int64_t rows, int64_t m) {
+  int best = 0;
+  double best_cost = 0.0;
+  for (int tile = 4; tile <= 32; tile += 4) {
+    const int64_t smem = tri_row_smem(m, tile);
+    if (smem > ctx->max_smem) break;
+    if (tile == 4 && tri_row_smem(m, 8) <= ctx->max_smem / 2) continue;
+    // 1 KB of an SM's shared memory goes to each CTA besides
+    const int64_t per_sm = std::min<int64_t>(32, (ctx->max_smem + 1024) / (smem + 1024));
+    const double rounds = (double)((rows + tile - 1) / tile) / (double)(per_sm * ctx->num_sms);
+    if (m > 1600 && rounds > 16.0) continue;
+    const double cost = std::ceil(rounds) + 0.25 * rounds + (form == 0 ? 0.01 : -0.01) * tile;
+    if (best == 0 || cost < best_cost) {
+      best = tile;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
+// Enqueues one batched solve on ctx->stream (device pointers).  Called with
+// ctx->mu held.  The kernel that reads rows in place takes its scratch from the
+// context's device pool (stream-ordered: every user of that pool runs on
+// ctx->stream).
 int tridag_launch(futhark_context* ctx, int form, int64_t rows, int64_t m, const float* a, const float* b,
                   const float* c, const float* y, float* out) {
   if (rows < 0 || m < 0 || m > INT32_MAX) return set_error(ctx, FUTHARK_PROGRAM_ERROR, "bad tridiagonal batch shape");
   if (rows == 0 || m == 0) return 0;
-  if (m <= kTriTmemMaxM && (m & 1) && rows % 4 == 0 && rows / 4 <= INT32_MAX - kTriTmaGroups) {
-    // odd m: inputs staged for the whole CTA by tensor copies of 4-system groups
-    const float* src[4] = {a, b, c, y};
-    bool ok = ctx->tri_map_rows == rows && ctx->tri_map_m == m;
-    for (int i = 0; i < 4 && ok; i++) ok = ctx->tri_map_src[i] == src[i];
-    if (!ok) {  // encode the maps of this batch (host work: reused while the batch repeats)
-      ok = true;
-      for (int i = 0; i < 4 && ok; i++) ok = tri_group_map(&ctx->tri_maps[i], src[i], rows, m);
-      ctx->tri_map_rows = ok ? rows : -1;
-      ctx->tri_map_m = ok ? m : -1;
-      for (int i = 0; i < 4; i++) ctx->tri_map_src[i] = ok ? src[i] : nullptr;
-    }
-    if (ok) {
-      const CUtensorMap* maps = ctx->tri_maps;
-      const int64_t nblk = (rows + 32 * kTriTmemWarps - 1) / (32 * kTriTmemWarps);
-      const int cols = tri_tmem_cols((int)m);
-      auto fk = cols == 256 ? (form == 0 ? lvc_tridag_tma_kernel<0, 256> : lvc_tridag_tma_kernel<1, 256>)
-                            : (form == 0 ? lvc_tridag_tma_kernel<0, 512> : lvc_tridag_tma_kernel<1, 512>);
-      const size_t smem = tri_tma_smem(cols);
-      if (int rc = tri_smem_limit(ctx, (const void*)fk, smem)) return rc;
-      fk<<<(unsigned)nblk, kTriTmaThreads, smem, ctx->stream>>>(maps[0], maps[1], maps[2], maps[3], rows,
-                                                                     (int)m, out);
-      const cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) return cuda_fail(ctx, e, "tridiagonal launch");
-      return 0;
-    }
-  }
-  if (m <= kTriTmemMaxM) {  // intermediates in tensor memory, four warps per CTA
-    const int64_t nblk = (rows + 32 * kTriTmemWarps - 1) / (32 * kTriTmemWarps);
+  if (const int tile = tri_row_tile(ctx, form, rows, m)) {
+    using Fn = void (*)(int64_t, int, int, const float*, const float*, const float*, const float*, float*, bool, bool);
+    static const Fn fns[2][3] = {{lvc_tridag_row_kernel<0, 1>, lvc_tridag_row_kernel<0, 2>, lvc_tridag_row_kernel<0, 4>},
+                                 {lvc_tridag_row_kernel<1, 1>, lvc_tridag_row_kernel<1, 2>, lvc_tridag_row_kernel<1, 4>}};
+    const Fn fn = fns[form == 0 ? 0 : 1][tri_row_vw(m) / 2];
+    const int64_t nblk = (rows + tile - 1) / tile;
     if (nblk > INT32_MAX) return set_error(ctx, FUTHARK_PROGRAM_ERROR, "tridiagonal batch too large");
-    const int cols = tri_tmem_cols((int)m);
-    auto fk = cols == 256 ? (form == 0 ? lvc_tridag_tmem_kernel<0, 256> : lvc_tridag_tmem_kernel<1, 256>)
-                          : (form == 0 ? lvc_tridag_tmem_kernel<0, 512> : lvc_tridag_tmem_kernel<1, 512>);
-    const size_t smem = tri_tmem_smem(cols);
-    if (int rc = tri_smem_limit(ctx, (const void*)fk, smem)) return rc;
-    fk<<<(unsigned)nblk, 32 * kTriTmemWarps, smem, ctx->stream>>>(rows, (int)m, a, b, c, y, out);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "tridiagonal launch");
-    return 0;
-  }
-  if (m <= kTriMaxM) {  // inputs streamed, intermediates in shared memory
-    const int64_t nblk = (rows + 31) / 32;
-    if (nblk > INT32_MAX) return set_error(ctx, FUTHARK_PROGRAM_ERROR, "tridiagonal batch too large");
-    const size_t smem = sizeof(float) * (size_t)tri_stream_floats((int)m);
-    const size_t smem_max = sizeof(float) * (size_t)tri_stream_floats(kTriMaxM);
-    auto fs = form == 0 ? lvc_tridag_stream_kernel<0> : lvc_tridag_stream_kernel<1>;
-    if (int rc = tri_smem_limit(ctx, (const void*)fs, smem_max)) return rc;
-    fs<<<(unsigned)nblk, 32, smem, ctx->stream>>>(rows, (int)m, a, b, c, y, out);
+    const auto aligned = [](const float* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    if (int rc = tri_smem_limit(ctx, (const void*)fn)) return rc;
+    fn<<<(unsigned)nblk, 32, (size_t)tri_row_smem(m, tile), ctx->stream>>>(
+        rows, (int)m, tile, a, b, c, y, out, aligned(a) && aligned(b) && aligned(c) && aligned(y), aligned(out));
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "tridiagonal launch");
     return 0;
