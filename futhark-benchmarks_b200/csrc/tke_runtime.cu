@@ -48,8 +48,10 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <type_traits>
 
 #include "tke.h"
+#include "exact_math.cuh"
 #include "fut_api.cuh"
 
 namespace {
@@ -390,115 +392,214 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
   float* q0 = p.q0 + col;
   float* q1 = p.q1 + col;
 
-  // Forward, staged a chunk of kColCh z at a time and computed one z at a
-  // time (a rolled loop: the unrolled chunk body cost more than its overlap
-  // of the coefficients of neighbouring z saved): (A) the coefficients
+  // Forward, staged a chunk of kColCh z at a time: (A) the coefficients
   // (tke.fut:103-210); (B) tridagPar's recurrences 1 (the 4-tuple scan for
   // b', tridiag.fut:9-33) and 2 (y', :38-56) folded left to right --
   // recurrence 2 at z needs b' of z - 1 only; (C) the two quotients the
   // backward recurrence folds.  Every lane runs A and B (the shuffles need
-  // the whole warp); only interior columns store.
-  float s0 = 1.0f, s1 = 0.0f, s2 = 0.0f, s3 = 1.0f, b0 = 0.0f, y0 = 0.0f, r0 = 0.0f, r1 = 1.0f;
-  float dm = 0.0f, cprev = 0.0f;
-  double rbpprev = 0.0;  // 1 / b' of z - 1 (DR_)
-  col_stage_chunk(p, st, col0, ncol, 0, lane);
-  cp_async_commit();
-  if (nch > 1) col_stage_chunk(p, st + kColStageFloats, col0, ncol, 1, lane);
-  cp_async_commit();
-  // the per-z constants of the next chunk, loaded a chunk ahead: lane l
-  // holds dzw and dzt of z + 1 for z = (chunk) * kColCh + l % kColCh
-  float dzN = 1.0f, dztN = 1.0f;
-  auto ld_consts = [&](int k) {
-    const int zl = k * kColCh + (lane & (kColCh - 1));
-    dzN = zl < Z ? p.dzw[zl] : 1.0f;
-    dztN = zl < Z - 1 ? p.dzt[zl + 1] : 1.0f;
-  };
-  ld_consts(0);
-  for (int k = 0; k < nch; k++) {
-    if (k + 2 < nch) col_stage_chunk(p, st + ((k + 2) % kColStages) * kColStageFloats, col0, ncol, k + 2, lane);
+  // the whole warp); only interior columns store.  The pass runs with near_div
+  // and its like, the coefficients of a chunk's z without a branch and ahead of
+  // the recurrences, and once more one z at a time with exact division where an
+  // interior column left their range.  (200 x 200 x 100 with sea floor at every
+  // depth: 130 -> 86 us for the kernel, which spent its time on the chain of each z,
+  // six divisions and their branches, at two warps per scheduler; what bounds it now
+  // is that chain and the instructions, half an issue slot per cycle.)
+  auto forward = [&](auto near) -> bool {
+    constexpr bool kNear = decltype(near)::value;
+    RangeCheck in;
+    float s0 = 1.0f, s1 = 0.0f, s2 = 0.0f, s3 = 1.0f, b0 = 0.0f, y0 = 0.0f, r0 = 0.0f, r1 = 1.0f;
+    float dm = 0.0f, cprev = 0.0f;
+    double rbpprev = 0.0;         // 1 / b' of z - 1 (DR_)
+    float bprev = 1.0f, rbprev = 1.0f;  // b' of z - 1 and its reciprocal (near_div)
+    col_stage_chunk(p, st, col0, ncol, 0, lane);
     cp_async_commit();
-    cp_async_wait_all_but_one();  // chunks k and k + 1 have landed
-    __syncwarp();
-    const float* cur = st + (k % kColStages) * kColStageFloats;
-    const float* nxt = st + ((k + 1) % kColStages) * kColStageFloats;
-    const int zbase = k * kColCh;
-    const int zn = min(kColCh, Z - zbase);
-    // the chunk's per-z constants, lane l holding those of z = zbase + l % kColCh
-    const float dz_l = dzN;
-    const float fac_l = zbase + (lane & (kColCh - 1)) < Z - 1 ? M_(M_(D_(kDtTke, dztN), kAlphaTke), 0.5f) : 0.0f;
-    const double rdz_l = Rd_(dz_l);  // the quotients by dz of the interior levels (DR_)
-    if (k + 1 < nch) ld_consts(k + 1);
+    if (nch > 1) col_stage_chunk(p, st + kColStageFloats, col0, ncol, 1, lane);
+    cp_async_commit();
+    // the per-z constants of the next chunk, loaded a chunk ahead: lane l
+    // holds dzw and dzt of z + 1 for z = (chunk) * kColCh + l % kColCh
+    float dzN = 1.0f, dztN = 1.0f;
+    auto ld_consts = [&](int k) {
+      const int zl = k * kColCh + (lane & (kColCh - 1));
+      dzN = zl < Z ? p.dzw[zl] : 1.0f;
+      dztN = zl < Z - 1 ? p.dzt[zl + 1] : 1.0f;
+    };
+    ld_consts(0);
+    for (int k = 0; k < nch; k++) {
+      if (k + 2 < nch) col_stage_chunk(p, st + ((k + 2) % kColStages) * kColStageFloats, col0, ncol, k + 2, lane);
+      cp_async_commit();
+      cp_async_wait_all_but_one();  // chunks k and k + 1 have landed
+      __syncwarp();
+      const float* cur = st + (k % kColStages) * kColStageFloats;
+      const float* nxt = st + ((k + 1) % kColStages) * kColStageFloats;
+      const int zbase = k * kColCh;
+      const int zn = min(kColCh, Z - zbase);
+      // the chunk's per-z constants, lane l holding those of z = zbase + l % kColCh
+      const float dz_l = dzN;
+      const float fac_l = zbase + (lane & (kColCh - 1)) < Z - 1 ? M_(M_(D_(kDtTke, dztN), kAlphaTke), 0.5f) : 0.0f;
+      if constexpr (kNear) {
+        // dz inside 2^-20 .. 2^20: what is divided by it below stays a dividend
+        const float rdz_l = near_rcp(dz_l);
+        in.divisor(M_(dz_l, dz_l));
+        if (k + 1 < nch) ld_consts(k + 1);
+        // (A) for the chunk's four z, independent of one another and of (B);
+        // selections instead of branches
+        float a_[kColCh], b_[kColCh], c_[kColCh], d_[kColCh];
+#pragma unroll
+        for (int zz = 0; zz < kColCh; zz++) {
+          const int z = zbase + zz;
+          const bool top = z == Z - 1;  // uniform
+          const float fac = __shfl_sync(kAll, fac_l, zz);
+          const float dz = __shfl_sync(kAll, dz_l, zz), rdz = __shfl_sync(kAll, rdz_l, zz);
+          const float dd = top ? M_(0.5f, dz) : dz, rdd = top ? M_(2.0f, rdz) : rdz;
+          const float t = cur[zz * kColPad + lane];
+          const float kap = cur[(kColCh + zz) * kColPad + lane];
+          const float fo = cur[(3 * kColCh + zz) * kColPad + lane];
+          const float kapn = zz + 1 < kColCh ? cur[(kColCh + zz + 1) * kColPad + lane] : nxt[kColCh * kColPad + lane];
+          const float d0 = z < Z - 1 ? M_(fac, A_(kap, kapn)) : 0.0f;  // delta (:103-108)
+          const bool edge = land && z == ks, water = land && z >= ks;
+          const float mx = water ? cur[(2 * kColCh + zz) * kColPad + lane] : 1.0f;
+          const float t0 = max_(0.0f, t), sq = near_sqrt(t0);
+          a_[zz] = !edge && water && z > 0 ? near_div(-dm, dd, rdd) : 0.0f;
+          // 1 + (delta of the levels around) / dz + dissipation: the edge has
+          // only the level above, the top only the one below and half a dz
+          const bool end = edge || top;
+          const float dsum = edge ? d0 : top ? dm : A_(d0, dm);
+          const float kc = M_(kDtTke, kCEps);
+          const float rest = M_(near_div(end ? kc : M_(kc, sq), mx, near_rcp(mx)), end ? sq : 1.0f);
+          b_[zz] = water ? A_(A_(1.0f, near_div(dsum, dd, rdd)), rest) : 1.0f;
+          c_[zz] = z < Z - 1 && water ? near_div(-d0, dz, rdz) : 0.0f;
+          const float tmp = A_(t, M_(kDtTke, fo));
+          d_[zz] = water ? tmp : 0.0f;
+          if (top && water) d_[zz] = A_(tmp, D_(M_(kDtTke, fts), M_(0.5f, dz)));
+          dm = d0;
+          if (zz < zn) {
+            in.divisor(mx);
+            in.dividend(t0);
+            in.dividend(d0);
+          }
+        }
+        // (B), (C)
+#pragma unroll
+        for (int zz = 0; zz < kColCh; zz++) {
+          if (zz >= zn) break;
+          float bp, yp;
+          if (zz == 0 && k == 0) {  // the neutral elements
+            b0 = b_[0];
+            y0 = d_[0];
+            bp = A_(b0, 0.0f);
+            yp = A_(0.0f, y0);
+          } else {
+            const float m1 = S_(0.0f, M_(a_[zz], cprev));
+            const float pz = M_(s0, b_[zz]);
+            const float value = near_rcp(pz);
+            const float n0 = M_(A_(pz, M_(m1, s2)), value);
+            const float n1 = M_(A_(M_(b_[zz], s1), M_(m1, s3)), value);
+            const float n2 = M_(s0, value);  // s0 + 0 * s2 is s0: pz is in range, so s0 is not zero and s2 finite
+            const float n3 = M_(A_(s1, M_(0.0f, s3)), value);
+            s0 = n0;
+            s1 = n1;
+            s2 = n2;
+            s3 = n3;
+            const float den = A_(M_(s2, b0), s3);
+            bp = near_div(A_(M_(s0, b0), s1), den, near_rcp(den));
+            const float l1 = S_(0.0f, near_div(a_[zz], bprev, rbprev));
+            r0 = A_(d_[zz], M_(l1, r0));
+            r1 = M_(r1, l1);
+            yp = A_(r0, M_(r1, y0));
+            in.divisor(pz);
+            in.divisor(den);
+          }
+          const float rb = near_rcp(bp);
+          in.divisor(bp);
+          in.dividend(yp);
+          cprev = c_[zz];
+          bprev = bp;
+          rbprev = rb;
+          if (inner) {
+            const int64_t o = (int64_t)(zbase + zz) * qs;
+            q0[o] = yp == 0.0f ? M_(yp, rb) : near_div(yp, bp, rb);
+            q1[o] = S_(0.0f, near_div(cprev, bp, rb));
+          }
+        }
+      } else {
+        const double rdz_l = Rd_(dz_l);  // the quotients by dz of the interior levels (DR_)
+        if (k + 1 < nch) ld_consts(k + 1);
 #pragma unroll 1
-    for (int zz = 0; zz < zn; zz++) {  // (A), (B), (C) for one z
-      const float fac = __shfl_sync(kAll, fac_l, zz);
-      const float dz = __shfl_sync(kAll, dz_l, zz);
-      const double rdz = __shfl_sync(kAll, rdz_l, zz);
-      const int z = zbase + zz;
-      const float t = cur[zz * kColPad + lane];
-      const float kap = cur[(kColCh + zz) * kColPad + lane];
-      const float mx = cur[(2 * kColCh + zz) * kColPad + lane];
-      const float fo = cur[(3 * kColCh + zz) * kColPad + lane];
-      const float kapn = zz + 1 < kColCh ? cur[(kColCh + zz + 1) * kColPad + lane] : nxt[kColCh * kColPad + lane];
-      const float d0 = z < Z - 1 ? M_(fac, A_(kap, kapn)) : 0.0f;  // delta (:103-108)
-      const bool edge = land && z == ks, water = land && z >= ks;
-      const float sq = __fsqrt_rn(max_(0.0f, t));
-      float a_ = 0.0f, b_ = 0.0f, c_ = 0.0f, d_ = 0.0f;
-      if (edge || !water) a_ = 0.0f;
-      else if (z > 0 && z < Z - 1) a_ = DR_(-dm, rdz);
-      else if (z == Z - 1) a_ = D_(-dm, M_(0.5f, dz));
-      if (!water) b_ = 1.0f;
-      else if (edge) b_ = A_(A_(1.0f, DR_(d0, rdz)), M_(__fdiv_rn(M_(kDtTke, kCEps), mx), sq));
-      else if (z > 0 && z < Z - 1) b_ = A_(A_(1.0f, DR_(A_(d0, dm), rdz)), __fdiv_rn(M_(M_(kDtTke, kCEps), sq), mx));
-      else if (z == Z - 1) b_ = A_(A_(1.0f, D_(dm, M_(0.5f, dz))), M_(D_(M_(kDtTke, kCEps), mx), sq));
-      if (z < Z - 1) c_ = water ? DR_(-d0, rdz) : 0.0f;
-      if (water) {
-        const float tmp = A_(t, M_(kDtTke, fo));
-        d_ = (z == Z - 1) ? A_(tmp, D_(M_(kDtTke, fts), M_(0.5f, dz))) : tmp;
+      for (int zz = 0; zz < zn; zz++) {  // (A), (B), (C) for one z
+        const float fac = __shfl_sync(kAll, fac_l, zz);
+        const float dz = __shfl_sync(kAll, dz_l, zz);
+        const double rdz = __shfl_sync(kAll, rdz_l, zz);
+        const int z = zbase + zz;
+        const float t = cur[zz * kColPad + lane];
+        const float kap = cur[(kColCh + zz) * kColPad + lane];
+        const float mx = cur[(2 * kColCh + zz) * kColPad + lane];
+        const float fo = cur[(3 * kColCh + zz) * kColPad + lane];
+        const float kapn = zz + 1 < kColCh ? cur[(kColCh + zz + 1) * kColPad + lane] : nxt[kColCh * kColPad + lane];
+        const float d0 = z < Z - 1 ? M_(fac, A_(kap, kapn)) : 0.0f;  // delta (:103-108)
+        const bool edge = land && z == ks, water = land && z >= ks;
+        const float sq = __fsqrt_rn(max_(0.0f, t));
+        float a_ = 0.0f, b_ = 0.0f, c_ = 0.0f, d_ = 0.0f;
+        if (edge || !water) a_ = 0.0f;
+        else if (z > 0 && z < Z - 1) a_ = DR_(-dm, rdz);
+        else if (z == Z - 1) a_ = D_(-dm, M_(0.5f, dz));
+        if (!water) b_ = 1.0f;
+        else if (edge) b_ = A_(A_(1.0f, DR_(d0, rdz)), M_(__fdiv_rn(M_(kDtTke, kCEps), mx), sq));
+        else if (z > 0 && z < Z - 1) b_ = A_(A_(1.0f, DR_(A_(d0, dm), rdz)), __fdiv_rn(M_(M_(kDtTke, kCEps), sq), mx));
+        else if (z == Z - 1) b_ = A_(A_(1.0f, D_(dm, M_(0.5f, dz))), M_(D_(M_(kDtTke, kCEps), mx), sq));
+        if (z < Z - 1) c_ = water ? DR_(-d0, rdz) : 0.0f;
+        if (water) {
+          const float tmp = A_(t, M_(kDtTke, fo));
+          d_ = (z == Z - 1) ? A_(tmp, D_(M_(kDtTke, fts), M_(0.5f, dz))) : tmp;
+        }
+        dm = d0;
+        float m0 = 1.0f, m1 = 0.0f, m2 = 0.0f, m3 = 1.0f;
+        if (z > 0) {
+          m0 = b_;
+          m1 = S_(0.0f, M_(a_, cprev));
+          m2 = 1.0f;
+          m3 = 0.0f;
+        } else {
+          b0 = b_;
+        }
+        const float value = __frcp_rn(M_(s0, m0));
+        const float n0 = M_(A_(M_(m0, s0), M_(m1, s2)), value);
+        const float n1 = M_(A_(M_(m0, s1), M_(m1, s3)), value);
+        const float n2 = M_(A_(M_(m2, s0), M_(m3, s2)), value);
+        const float n3 = M_(A_(M_(m2, s1), M_(m3, s3)), value);
+        s0 = n0;
+        s1 = n1;
+        s2 = n2;
+        s3 = n3;
+        // (quotients whose dividend is rarely zero skip D_'s test for one)
+        const float bpz = __fdiv_rn(A_(M_(s0, b0), s1), A_(M_(s2, b0), s3));
+        const double rbp = Rd_(bpz);  // three quotients by b'_z: y'_z, c_z here, a_{z+1} next
+        float l0 = 0.0f, l1 = 1.0f;
+        if (z > 0) {
+          l0 = d_;
+          l1 = S_(0.0f, DR_(a_, rbpprev));
+        } else {
+          y0 = d_;
+        }
+        const float rn0 = A_(l0, M_(l1, r0)), rn1 = M_(r1, l1);
+        r0 = rn0;
+        r1 = rn1;
+        const float ypz = A_(r0, M_(r1, y0));
+        cprev = c_;
+        rbpprev = rbp;
+        if (inner) {
+          const int64_t o = (int64_t)z * qs;
+          q0[o] = DR_(ypz, rbp);
+          q1[o] = S_(0.0f, DR_(c_, rbp));
+        }
       }
-      dm = d0;
-      float m0 = 1.0f, m1 = 0.0f, m2 = 0.0f, m3 = 1.0f;
-      if (z > 0) {
-        m0 = b_;
-        m1 = S_(0.0f, M_(a_, cprev));
-        m2 = 1.0f;
-        m3 = 0.0f;
-      } else {
-        b0 = b_;
       }
-      const float value = __frcp_rn(M_(s0, m0));
-      const float n0 = M_(A_(M_(m0, s0), M_(m1, s2)), value);
-      const float n1 = M_(A_(M_(m0, s1), M_(m1, s3)), value);
-      const float n2 = M_(A_(M_(m2, s0), M_(m3, s2)), value);
-      const float n3 = M_(A_(M_(m2, s1), M_(m3, s3)), value);
-      s0 = n0;
-      s1 = n1;
-      s2 = n2;
-      s3 = n3;
-      // (quotients whose dividend is rarely zero skip D_'s test for one)
-      const float bpz = __fdiv_rn(A_(M_(s0, b0), s1), A_(M_(s2, b0), s3));
-      const double rbp = Rd_(bpz);  // three quotients by b'_z: y'_z, c_z here, a_{z+1} next
-      float l0 = 0.0f, l1 = 1.0f;
-      if (z > 0) {
-        l0 = d_;
-        l1 = S_(0.0f, DR_(a_, rbpprev));
-      } else {
-        y0 = d_;
-      }
-      const float rn0 = A_(l0, M_(l1, r0)), rn1 = M_(r1, l1);
-      r0 = rn0;
-      r1 = rn1;
-      const float ypz = A_(r0, M_(r1, y0));
-      cprev = c_;
-      rbpprev = rbp;
-      if (inner) {
-        const int64_t o = (int64_t)z * qs;
-        q0[o] = DR_(ypz, rbp);
-        q1[o] = S_(0.0f, DR_(c_, rbp));
-      }
+      __syncwarp();  // the next iteration refills this chunk's stage
     }
-    __syncwarp();  // the next iteration refills this chunk's stage
-  }
-  cp_async_wait_all();
+    cp_async_wait_all();
+    return !inner || in.ok(0x1p-60f);
+  };
+  if (!__all_sync(kAll, forward(std::true_type()))) forward(std::false_type());  // again, for any values
+  float r0, r1;
 
   // Backward, a chunk at a time from the top: recurrence 3 down the column
   // into the tile, then the chunk's cells (coalesced): take the solution or
