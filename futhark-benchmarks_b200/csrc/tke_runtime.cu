@@ -35,10 +35,8 @@
 // Every operation is explicitly rounded (no fused multiply-add) in the
 // reference's operand order -- the fold order of each recurrence included --
 // so the outputs equal the CPU oracle's, which reproduces the reference's
-// golden outputs, bit for bit.  Quotients by a divisor that stays fixed over
-// many of them (dz of a level, cos * dy of a row, cos * dx of a step) come
-// from its double reciprocal (DR_), which gives the same correctly rounded
-// float as the division.
+// golden outputs, bit for bit.  Divisions and square roots are corrected
+// approximations (exact_math.cuh) wherever the operands are in their range.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -110,14 +108,11 @@ __device__ __forceinline__ bool interior(const TkeArgs& p, int x, int y) {
 __device__ __forceinline__ float limiter(float cr) {
   return max_(0.0f, max_(min_(1.0f, M_(2.0f, cr)), min_(2.0f, cr)));
 }
-// uCFL is |scaledVel dt_tracer / dx|: from dx itself (RECIP false) or from
-// its double reciprocal rdx (RECIP true, DR_)
-template <bool RECIP>
-__device__ __forceinline__ float calcflux(float velfac, float velS, float dt_tracer, float dx, double rdx,
-                                          float varS, float varSM1, float varSP1, float varSP2, float maskS,
-                                          float maskSM1, float maskSP1) {
+// The flux for any values.
+__device__ __noinline__ float calcflux(float velfac, float velS, float dx, float varS, float varSM1, float varSP1,
+                                       float varSP2, float maskS, float maskSM1, float maskSP1) {
   const float scaledVel = M_(velfac, velS);
-  const float uCFL = fabsf(RECIP ? DR_(M_(scaledVel, dt_tracer), rdx) : D_(M_(scaledVel, dt_tracer), dx));
+  const float uCFL = fabsf(D_(M_(scaledVel, kDtTracer), dx));
   const float rjp = M_(S_(varSP2, varSP1), maskSP1);
   const float rj = M_(S_(varSP1, varS), maskS);
   const float rjm = M_(S_(varS, varSM1), maskSM1);
@@ -128,6 +123,34 @@ __device__ __forceinline__ float calcflux(float velfac, float velS, float dt_tra
   return S_(M_(M_(scaledVel, A_(varSP1, varS)), 0.5f),
             M_(M_(M_(fabsf(scaledVel), A_(S_(1.0f, cr), M_(uCFL, cr))), rj), 0.5f));
 }
+// The same through near_div, with rdx = 1 / dx correctly rounded and dx inside
+// 2^-20 .. 2^20; calcflux where an operand is too large for it.  Small ones need no
+// test.  The limiter's divisor is at least 1e-20 in magnitude.  A dividend below
+// 2^-103, where its quotient may not be the correctly rounded one, gives |cr| <
+// 2^-36, and with uCFL < 2^10 both 1 - cr and the sum with uCFL cr are then 1
+// whatever its last bits.  A velocity below 2^-103 gives uCFL < 2^-83, which counts
+// only beside 1 - cr = 0, and there its product with the velocity underflows to
+// zero.
+__device__ __forceinline__ float near_flux(float velfac, float velS, float dx, float rdx, float varS, float varSM1,
+                                           float varSP1, float varSP2, float maskS, float maskSM1, float maskSP1) {
+  const float scaledVel = M_(velfac, velS);
+  const float uCFL = fabsf(near_div(M_(scaledVel, kDtTracer), dx, rdx));
+  const float rj = M_(S_(varSP1, varS), maskS);
+  const float rjx = velS > 0.0f ? M_(S_(varS, varSM1), maskSM1) : M_(S_(varSP2, varSP1), maskSP1);
+  const float epsilon = 0.00000000000000000001f;
+  const float divisor = (fabsf(rj) < epsilon) ? epsilon : rj;
+  const float cr = limiter(near_div(rjx, divisor, near_rcp(divisor)));
+  const float flux = S_(M_(M_(scaledVel, A_(varSP1, varS)), 0.5f),
+                        M_(M_(M_(fabsf(scaledVel), A_(S_(1.0f, cr), M_(uCFL, cr))), rj), 0.5f));
+  if (fmaxf(fmaxf(fabsf(rj), fabsf(rjx)), fabsf(scaledVel)) < 0x1p40f && uCFL < 0x1p10f) return flux;
+  return calcflux(velfac, velS, dx, varS, varSM1, varSP1, varSP2, maskS, maskSM1, maskSP1);
+}
+// a / b, rb = 1 / b correctly rounded, b inside 2^-20 .. 2^20.
+__device__ __forceinline__ float near_quotient(float a, float b, float rb) {
+  const float q = near_div(a, b, rb);
+  return fabsf(a) > 0x1p-100f && fabsf(a) < 0x1p100f ? q : D_(a, b);
+}
+__device__ __forceinline__ bool near_divisor(float b) { return fabsf(b) > 0x1p-20f && fabsf(b) < 0x1p20f; }
 
 // lateral diffusion fluxes (:236-251), from tketau
 __device__ __forceinline__ float diff_east(const TkeArgs& p, int x, int y, int z) {
@@ -147,10 +170,8 @@ __device__ __forceinline__ float adv_east(const TkeArgs& p, int x, int y, int z)
   const float dx = M_(p.cost[y], p.dxt[x]);
   const float mWm1 = p.maskW[i3(p, x - 1, y, z)], mWs = p.maskW[i], mWp1 = p.maskW[i3(p, x + 1, y, z)],
               mWp2 = p.maskW[i3(p, x + 2, y, z)];
-  const bool in = x < p.X - 1;
-  return calcflux<false>(1.0f, p.utau[i], kDtTracer, dx, 0.0, p.tketau[i], p.tketau[i3(p, x - 1, y, z)],
-                  p.tketau[i3(p, x + 1, y, z)], p.tketau[i3(p, x + 2, y, z)], in ? M_(mWs, mWp1) : 0.0f,
-                  in ? M_(mWm1, mWs) : 0.0f, in ? M_(mWp1, mWp2) : 0.0f);
+  return calcflux(1.0f, p.utau[i], dx, p.tketau[i], p.tketau[i3(p, x - 1, y, z)], p.tketau[i3(p, x + 1, y, z)],
+                  p.tketau[i3(p, x + 2, y, z)], M_(mWs, mWp1), M_(mWm1, mWs), M_(mWp1, mWp2));
 }
 // ---------------------------------------------------------------------------
 // tke_advect_kernel
@@ -172,10 +193,14 @@ constexpr int kAdvThreads = 256;  // at <= 64 registers two CTAs fit beside two 
 // (rather than runs of consecutive (y, z)) keep most north neighbours in the
 // block when zdim is large: with zdim = 100, 2.56 rows of 256 threads held
 // none of them.
+// Issue-bound: 73 M warp instructions at 200 x 200 x 100 with divisions as the
+// compiler makes them and 64-bit indices, 93 us; near_flux and Ix leave 79 us.
+// Ix: the type of a cell's index, int32_t where the last one fits.
+template <typename Ix>
 __global__ void __launch_bounds__(kAdvThreads, 4) tke_advect_kernel(TkeArgs p, int xseg, int ty, int tz, int nzt) {
   __shared__ float sT[kAdvThreads], sW[kAdvThreads], sfn[kAdvThreads], sft[kAdvThreads];
   const int t = threadIdx.x;
-  const int64_t plane = (int64_t)p.Y * p.Z;
+  const Ix plane = (Ix)p.Y * p.Z;
   const int Z = p.Z;
   // position in the tile: the halo row in warp 0 (lanes 0 .. tz - 1), rows
   // 1 .. ty - 1 packed from thread 32 on, so the halo row's warp evaluates
@@ -191,7 +216,7 @@ __global__ void __launch_bounds__(kAdvThreads, 4) tke_advect_kernel(TkeArgs p, i
   const bool live = ry < ty && rz < tz && yy >= 0 && yy < p.Y && zz >= 0 && zz < Z;
   const bool owned = live && ry >= 1 && rz >= 1;
   const int y = live ? yy : 0, z = live ? zz : 0;
-  const int64_t qi = (int64_t)y * Z + z;
+  const Ix qi = (Ix)y * Z + z;
   const int xs = blockIdx.y * xseg, xe = min(p.X, xs + xseg);
   const bool n_in = ry >= 1 && ry + 2 < ty;  // (y - 1 .. y + 2, z) in this tile
   const int nm = ry == 1 ? t - 32 : t - tz, np1 = hwarp ? t + 32 : t + tz;  // threads of rows y - 1, y + 1
@@ -199,8 +224,11 @@ __global__ void __launch_bounds__(kAdvThreads, 4) tke_advect_kernel(TkeArgs p, i
   const bool yint = y >= 2 && y < p.Y - 2;
   const float cy = live ? p.cost[y] : 1.0f, cuy = live ? p.cosu[y] : 1.0f, dyt = live ? p.dyt[y] : 1.0f;
   const float dz = live ? p.dzw[z] : 1.0f;
-  // the divisors that stay fixed along x, as double reciprocals (DR_)
-  const double rdy = Rd_(M_(cy, dyt)), rdz = Rd_(dz), rhdz = Rd_(M_(0.5f, dz));
+  // the divisors that stay fixed along x, and their reciprocals where near_div
+  // takes them; dtketau's last quotient is by half a dz at the top
+  const float dyc = M_(cy, dyt), dtop = z == Z - 1 ? M_(0.5f, dz) : dz;
+  const bool near_yz = near_divisor(dyc) && near_divisor(dz) && near_divisor(dtop);
+  const float rdy = near_rcp(dyc), rdz = near_rcp(dz), rdtop = near_rcp(dtop);
   auto ldT = [&](int xx) { return (live && xx >= 0 && xx < p.X) ? p.tketau[xx * plane + qi] : 0.0f; };
   auto ldW = [&](int xx) { return (live && xx >= 0 && xx < p.X) ? p.maskW[xx * plane + qi] : 0.0f; };
   float T0 = ldT(xs - 1), T1 = ldT(xs), T2 = ldT(xs + 1), T3 = ldT(xs + 2);  // x - 1 .. x + 2
@@ -210,7 +238,7 @@ __global__ void __launch_bounds__(kAdvThreads, 4) tke_advect_kernel(TkeArgs p, i
   auto ldU = [&](const float* f, int xx) { return (live && xx < xe) ? f[xx * plane + qi] : 0.0f; };
   float uN = ldU(p.utau, xs), vN = ldU(p.vtau, xs), wN = ldU(p.wtau, xs);
   for (int x = xs; x < xe; x++) {
-    const int64_t i = x * plane + qi;
+    const Ix i = x * plane + qi;
     sT[t] = T1;
     sW[t] = W1;
     const float nT = ldT(x + 3), nW = ldW(x + 3);  // next step's window end
@@ -220,13 +248,17 @@ __global__ void __launch_bounds__(kAdvThreads, 4) tke_advect_kernel(TkeArgs p, i
     wN = ldU(p.wtau, x + 1);
     __syncthreads();
     float fe = 0.0f, fn = 0.0f, ft = 0.0f;
-    const double rdx = Rd_(M_(cy, p.dxt[x]));  // the east divisor of this x, for fe and dtketau
+    const float dxc = M_(cy, p.dxt[x]), rdx = near_rcp(dxc);  // the east divisor of this x, for fe and dtketau
+    const bool near = near_yz && near_divisor(dxc);
+    auto flux = [&](float velfac, float vel, float dx, float rdx_, float s_, float m1, float p1, float p2, float ms,
+                    float mm1, float mp1) {
+      return near ? near_flux(velfac, vel, dx, rdx_, s_, m1, p1, p2, ms, mm1, mp1)
+                  : calcflux(velfac, vel, dx, s_, m1, p1, p2, ms, mm1, mp1);
+    };
     if (live) {
       const bool xint = x >= 2 && x < p.X - 2;
       if (!hwarp && x >= 1 && x < p.X - 2 && yint) {
-        const bool in = x < p.X - 1;
-        fe = calcflux<true>(1.0f, uC, kDtTracer, 0.0f, rdx, T1, T0, T2, T3, in ? M_(W1, W2) : 0.0f,
-                      in ? M_(W0, W1) : 0.0f, in ? M_(W2, W3) : 0.0f);
+        fe = flux(1.0f, uC, dxc, rdx, T1, T0, T2, T3, M_(W1, W2), M_(W0, W1), M_(W2, W3));
       }
       if (y >= 1 && y < p.Y - 2 && xint) {
         float tm, tp1, tp2, wm, wp1, wp2;
@@ -245,9 +277,7 @@ __global__ void __launch_bounds__(kAdvThreads, 4) tke_advect_kernel(TkeArgs p, i
           wp1 = p.maskW[i + Z];
           wp2 = p.maskW[i + 2 * Z];
         }
-        const bool in = y < p.Y - 1;
-        fn = calcflux<true>(cuy, vC, kDtTracer, 0.0f, rdy, T1, tm, tp1, tp2, in ? M_(W1, wp1) : 0.0f,
-                      in ? M_(wm, W1) : 0.0f, in ? M_(wp1, wp2) : 0.0f);
+        fn = flux(cuy, vC, dyc, rdy, T1, tm, tp1, tp2, M_(W1, wp1), M_(wm, W1), M_(wp1, wp2));
       }
       if (!hwarp && z < Z - 1 && xint && yint) {
         float tm = 0.0f, tp1, tp2 = 0.0f, wm = 0.0f, wp1, wp2 = 0.0f;
@@ -274,7 +304,7 @@ __global__ void __launch_bounds__(kAdvThreads, 4) tke_advect_kernel(TkeArgs p, i
             wp2 = p.maskW[i + 2];
           }
         }
-        ft = calcflux<true>(1.0f, wC, kDtTracer, 0.0f, rdz, T1, tm, tp1, tp2, M_(W1, wp1), M_(wm, W1), M_(wp1, wp2));
+        ft = flux(1.0f, wC, dz, rdz, T1, tm, tp1, tp2, M_(W1, wp1), M_(wm, W1), M_(wp1, wp2));
       }
     }
     sfn[t] = fn;
@@ -282,15 +312,12 @@ __global__ void __launch_bounds__(kAdvThreads, 4) tke_advect_kernel(TkeArgs p, i
     __syncthreads();
     if (owned) {  // dtketau (:320-340)
       const float fnm = sfn[nm];  // the north flux of (y - 1, z): 0 outside the domain
-      const float ftm = sft[t - 1];   // the top flux of (y, z - 1)
-      float tmp;
-      if (x >= 2 && x < p.X - 2 && yint)
-        tmp = M_(W1, S_(DR_(-S_(fe, fe_prev), rdx), DR_(S_(fn, fnm), rdy)));
-      else
-        tmp = p.dtketau[i];
-      const float z0 = z == 0 ? S_(tmp, DR_(ft, rdz)) : tmp;
-      const float zm = (z >= 1 && z < Z - 1) ? S_(z0, DR_(S_(ft, ftm), rdz)) : z0;
-      p.dtketau_out[i] = (z == Z - 1) ? S_(zm, DR_(S_(ft, ftm), rhdz)) : zm;
+      const float ftm = z == 0 ? 0.0f : sft[t - 1];  // the top flux of (y, z - 1)
+      auto quot = [&](float a, float b, float rb) { return near ? near_quotient(a, b, rb) : D_(a, b); };
+      const float tmp = x >= 2 && x < p.X - 2 && yint
+                            ? M_(W1, S_(quot(-S_(fe, fe_prev), dxc, rdx), quot(S_(fn, fnm), dyc, rdy)))
+                            : p.dtketau[i];
+      p.dtketau_out[i] = S_(tmp, quot(S_(ft, ftm), dtop, rdtop));
     }
     fe_prev = fe;
     T0 = T1;
@@ -806,8 +833,9 @@ int step_launch(futhark_context* ctx, const tke_step_args* q) {
   const int64_t segs = (X + xseg - 1) / xseg;
   if (plane_blocks > INT32_MAX || segs > 65535)
     return set_error(ctx, FUTHARK_PROGRAM_ERROR, "tke step: plane too large");
-  tke_advect_kernel<<<dim3((unsigned)plane_blocks, (unsigned)segs), kAdvThreads, 0, ctx->aux>>>(p, xseg, (int)ty,
-                                                                                                (int)tz, (int)nzt);
+  const auto advect = n <= INT32_MAX ? tke_advect_kernel<int32_t> : tke_advect_kernel<int64_t>;
+  advect<<<dim3((unsigned)plane_blocks, (unsigned)segs), kAdvThreads, 0, ctx->aux>>>(p, xseg, (int)ty, (int)tz,
+                                                                                    (int)nzt);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(ctx, e, "tke advection launch");
   e = cudaEventRecord(ctx->ev_join, ctx->aux);
