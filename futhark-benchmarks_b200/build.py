@@ -34,7 +34,7 @@ HEADERS = ["lvc_kernels.cuh", "lvc_layout.h", "lvc_probe.cuh", "lvc_line.cuh", "
 TKE_SOURCES = ["tke_runtime.cu"]
 TKE_HEADERS = ["exact_math.cuh", "fut_api.cuh"]
 OP_SOURCES = ["op_runtime.cu"]
-OP_HEADERS = ["fut_api.cuh"]
+OP_HEADERS = ["exact_math.cuh", "fut_api.cuh"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-lineinfo", "-std=c++17",

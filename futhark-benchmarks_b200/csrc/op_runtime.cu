@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "op.h"
+#include "exact_math.cuh"
 #include "fut_api.cuh"
 
 namespace {
@@ -89,24 +90,27 @@ __constant__ float kTailB[8] = {1.0f, 0.59983220655588793769f, 0.136929880922735
                                 7.868691311456132591e-4f, 1.8463183175100546818e-5f, 1.4215117583164458887e-7f,
                                 2.04426310338993978564e-5f};
 
-// :52-57
+// :52-57.  near_div's range holds at every argument the Gaussian has: both
+// polynomials lie between 0.5 and 2^10 there (central branch: x in 0 .. 0.181;
+// tails: x in -0.24 .. 3.4 and 0 ..), and a NaN or infinite argument (a Sobol
+// integer of 0 or 2^B) gives NaN either way.
 __device__ __forceinline__ float poly_appr(float x, const float* a, const float* b) {
   const float num = x * (x * (x * (x * (x * (x * (x * a[7] + a[6]) + a[5]) + a[4]) + a[3]) + a[2]) + a[1]) + a[0];
   const float den = x * (x * (x * (x * (x * (x * (x * b[7] + b[6]) + b[5]) + b[4]) + b[3]) + b[2]) + b[1]) + b[0];
-  return num / den;
+  return near_div(num, den, near_rcp(den));
 }
 
 // :120-136, split at its branch: gauss_central for |p - 0.5| <= 0.425,
 // gauss_tail otherwise
 __device__ __forceinline__ bool gauss_is_central(float dp) {
-  return (dp < 0.0f && 0.0f - dp <= 0.425f) || (0.0f <= dp && dp <= 0.425f);
+  return fabsf(dp) <= 0.425f;
 }
 __device__ __forceinline__ float gauss_central(float dp) {
   return dp * poly_appr(0.180625f - dp * dp, kSmallA, kSmallB);
 }
 __device__ __forceinline__ float gauss_tail(float dp) {
   const float pp = dp < 0.0f ? dp + 0.5f : 0.5f - dp;
-  const float r = sqrtf(-f32log(pp));
+  const float r = near_sqrt(-f32log(pp));  // 1.6 .. 4.8, or infinite or NaN: then so is x
   const float x = r <= 5.0f ? poly_appr(r - 1.6f, kInterA, kInterB) : poly_appr(r - 5.0f, kTailA, kTailB);
   return dp < 0.0f ? 0.0f - x : x;
 }
@@ -154,7 +158,7 @@ __global__ void __launch_bounds__(kOpThreads, OpShape<C>::kMinCtas) op_paths_ker
   const int64_t lo = N * t / T, hi = N * (t + 1) / T;
   const int B = a.num_bits;
   const uint32_t bits = B >= 32 ? 0xffffffffu : ((1u << B) - 1u);
-  const float divisor = ldexpf(1.0f, B);  // 2 ** num_bits, exact
+  const float scale = ldexpf(1.0f, -B);  // x / 2 ** num_bits is x * 2 ** -num_bits, both exact
   const int nm = min(kOpModels, a.num_models - m0);
   double acc[kOpModels];
 #pragma unroll
@@ -177,11 +181,11 @@ __global__ void __launch_bounds__(kOpThreads, OpShape<C>::kMinCtas) op_paths_ker
     // Brownian bridge per underlying (:142-175), Gaussians on the fly
     for (int k = 0; k < K; k++) bb[k] = 0.0f;
     for (int u = 0; u < U; u++) {
-      bb[(s_ind[0] - 1) * U + u] = s_dat[0] * ugaussian_el((float)xs[u] / divisor);
+      bb[(s_ind[0] - 1) * U + u] = s_dat[0] * ugaussian_el((float)xs[u] * scale);
       for (int i = 1; i < D; i++) {
         const int j = s_ind[D + i] - 1, kk = s_ind[2 * D + i] - 1, l = s_ind[i] - 1;
         const float wk = bb[kk * U + u];
-        const float zi = ugaussian_el((float)xs[i * U + u] / divisor);
+        const float zi = ugaussian_el((float)xs[i * U + u] * scale);
         const float tmp = s_dat[2 * D + i] * wk + s_dat[i] * zi;
         bb[l * U + u] = j == -1 ? tmp : tmp + s_dat[D + i] * bb[j * U + u];
       }
@@ -372,7 +376,7 @@ __global__ void __launch_bounds__(kWarpPathWarps * 32, 2) op_paths_warp_kernel(O
   const int64_t lo = N * w / W, hi = N * (w + 1) / W;
   const int B = a.num_bits;
   const uint32_t bits = B >= 32 ? 0xffffffffu : ((1u << B) - 1u);
-  const float divisor = ldexpf(1.0f, B);
+  const float scale = ldexpf(1.0f, -B);
   const int nm = min(kOpModels, a.num_models - m0);
   double acc[kOpModels];
 #pragma unroll
@@ -402,7 +406,7 @@ __global__ void __launch_bounds__(kWarpPathWarps * 32, 2) op_paths_warp_kernel(O
       const int k = k0 + lane;
       bool tail = false;
       if (k < K) {
-        const float dp = (float)sX[k] / divisor - 0.5f;
+        const float dp = (float)sX[k] * scale - 0.5f;
         if (gauss_is_central(dp)) sG[k] = gauss_central(dp);
         else tail = true;
       }
@@ -413,7 +417,7 @@ __global__ void __launch_bounds__(kWarpPathWarps * 32, 2) op_paths_warp_kernel(O
     __syncwarp();
     for (int q = lane; q < nq; q += 32) {
       const int k = queue[q];
-      sG[k] = gauss_tail((float)sX[k] / divisor - 0.5f);
+      sG[k] = gauss_tail((float)sX[k] * scale - 0.5f);
     }
     __syncwarp();
     for (int k = lane; k < K; k += 32) sB[k] = 0.0f;
