@@ -338,9 +338,12 @@ __global__ void op_transpose_dirs_kernel(const int32_t* __restrict__ dir_vs, int
   }
 }
 
+// *taken != 0: op_paths_block_kernel has priced the paths.
 template <int C>
 __global__ void __launch_bounds__(kWarpPathWarps * 32, 2) op_paths_warp_kernel(OpDev a, const int32_t* __restrict__ dirT,
-                                                                            int m0, double* __restrict__ partial) {
+                                                                            int m0, double* __restrict__ partial,
+                                                                            const int* __restrict__ taken) {
+  if (*taken) return;
   using L = OpWarpSmem<C>;
   constexpr int D = OpShape<C>::D, U = OpShape<C>::U, K = D * U, KP = L::KP;
   constexpr unsigned kAll = 0xffffffffu;
@@ -520,6 +523,302 @@ __global__ void __launch_bounds__(kWarpPathWarps * 32, 2) op_paths_warp_kernel(O
       partial[(int64_t)mm * gridDim.x + blockIdx.x] = sum;
     }
     __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// CTA per 32 paths (contract 3), for a bridge in which every step fills a date of
+// its own from dates filled before -- what a Brownian bridge is; other index
+// patterns are left to op_paths_warp_kernel.
+// ---------------------------------------------------------------------------
+// The bridge is then done in place: the Gaussian of step i waits in the slot of
+// the date that step i fills, so one [date][underlying][path] array holds the
+// paths (145 KB of shared memory), and every phase runs with all 32 lanes busy:
+//   Gaussians   lane = dimension, a warp walking 8 paths of 32 dimensions: the
+//               next path's Sobol integer is one XOR (Gray code); tail arguments
+//               are queued per warp and evaluated 32 at a time
+//   bridge      lane = path, the steps of a level spread over the warps
+//   prices      lane = path: all warps but the last compute the exponentials
+//               of a chunk of dates, while the last multiplies up and tests the
+//               chunk before it, date by date
+// A warp per path with its lanes over the dimensions spent 13 K warp instructions
+// per path, a third of them on steps with few lanes busy (the bridge's levels, the
+// product on 3 lanes); this spends 7 K, half in the Gaussians and a third in the
+// exponentials, and is bound by issuing them.  131072 paths: 2531 us there, 1183
+// here; 2048: 144 and 64; 20 warps, the most with 87 registers each (16 1236, 24
+// 1188, 32 with spills 1283).
+constexpr int kBlkWarps = 20, kBlkThreads = 32 * kBlkWarps;
+constexpr int kBlkRuns = 8;    // paths of a Gaussian item
+constexpr int kBlkDates = 57;  // dates of a chunk: three per computing warp
+
+struct OpBlk {
+  static constexpr int D = OpShape<3>::D, U = OpShape<3>::U, K = D * U;
+  static constexpr int PS = 33;                                 // stride of a slot's 32 paths
+  static constexpr int oB = 0;                                  // [K][PS] Gaussians, then the bridge
+  static constexpr int oE = oB + (K * PS + 3) / 4 * 4;          // [2][kBlkDates][U][32] exponentials
+  static constexpr int oBase = oE + 2 * kBlkDates * U * 32;     // [K] Sobol integers of the block's path 0
+  static constexpr int oStep = oBase + (K + 3) / 4 * 4;         // [D] of l, k, j, sd | rw, lw: steps by level
+  static constexpr int oStep2 = oStep + 4 * D;
+  static constexpr int oStart = oStep2 + (2 * D + 3) / 4 * 4;   // [D + 2]
+  static constexpr int oSlot = oStart + D + 2;                  // [D] date of step i
+  static constexpr int oQueue = oSlot + D;                      // [kBlkWarps][64] arguments, then slots
+  static constexpr int kWords = oQueue + kBlkWarps * 128;
+  // the schedule's scratch, in B's place
+  static constexpr int oWriter = oB, oLevel = oB + D, oCount = oB + 2 * D;
+};
+
+// Levels of the bridge's steps -- one more than those of the steps that filled the
+// dates it reads -- and the steps sorted by level; false if a step fills a date
+// twice or reads one not filled before it.  All threads of the CTA.
+__device__ bool op_block_schedule(const int32_t* __restrict__ ind, const float* __restrict__ dat, float* sm,
+                                  int& nlev) {
+  using L = OpBlk;
+  constexpr int D = L::D;
+  const int i = threadIdx.x;
+  static_assert(D <= kBlkThreads, "a thread per step");
+  int* writer = reinterpret_cast<int*>(sm) + L::oWriter;
+  int* level = reinterpret_cast<int*>(sm) + L::oLevel;
+  int* count = reinterpret_cast<int*>(sm) + L::oCount;
+  int* start = reinterpret_cast<int*>(sm) + L::oStart;
+  int* slot = reinterpret_cast<int*>(sm) + L::oSlot;
+  const bool step = i < D;
+  const int l = step ? ind[i] - 1 : 0, j = step && i > 0 ? ind[D + i] - 1 : -1, k = step && i > 0 ? ind[2 * D + i] - 1 : 0;
+  bool good = l >= 0 && l < D && j >= -1 && j < D && k >= 0 && k < D;
+  if (step) writer[i] = D;
+  __syncthreads();
+  if (step && good && atomicMin(&writer[l], i) != D) good = false;
+  if (step) {
+    level[i] = 0;
+    count[i] = 0;
+    slot[i] = l;
+  }
+  if (!__syncthreads_and(good)) return false;
+  // every date has its one writer: D steps, no date twice
+  const int wk = step && i > 0 ? writer[k] : -1, wj = j >= 0 ? writer[j] : -1;
+  if (!__syncthreads_and(!(step && i > 0) || (wk < i && wj < i))) return false;
+  int lev = 0;
+  for (bool moved = true; moved;) {  // as many rounds as there are levels
+    int now = lev;
+    if (step && i > 0) now = max(level[wk], wj >= 0 ? level[wj] : 0) + 1;
+    moved = __syncthreads_or(now != lev);
+    lev = now;
+    if (step) level[i] = lev;
+    __syncthreads();
+  }
+  int rank = 0;
+  if (step && i > 0) rank = atomicAdd(&count[lev], 1);
+  __syncthreads();
+  if (i == 0) {
+    int at = 0, v = 1;
+    start[0] = start[1] = 0;
+    for (; v < D && count[v] > 0; v++) start[v + 1] = at += count[v];
+    start[D + 1] = v - 1;
+  }
+  __syncthreads();
+  nlev = start[D + 1];
+  if (step && i > 0) {
+    const int at = start[lev] + rank;
+    int* s4 = reinterpret_cast<int*>(sm) + L::oStep + 4 * at;
+    s4[0] = l * L::U * L::PS;
+    s4[1] = k * L::U * L::PS;
+    s4[2] = j < 0 ? -1 : j * L::U * L::PS;
+    sm[L::oStep + 4 * at + 3] = dat[i];
+    sm[L::oStep2 + 2 * at] = dat[2 * D + i];
+    sm[L::oStep2 + 2 * at + 1] = dat[D + i];
+  }
+  __syncthreads();
+  return true;
+}
+
+// partial: [models of the launch][slots], this kernel's sums first, zeros after;
+// *taken: whether this kernel priced the paths.
+__global__ void __launch_bounds__(kBlkThreads, 1) op_paths_block_kernel(OpDev a, const int32_t* __restrict__ dirT,
+                                                                       int m0, double* __restrict__ partial, int slots,
+                                                                       int* __restrict__ taken) {
+  using L = OpBlk;
+  constexpr int D = L::D, U = L::U, K = L::K, PS = L::PS;
+  constexpr unsigned kAll = 0xffffffffu;
+  extern __shared__ __align__(16) float op_dyn[];
+  float* const B_ = op_dyn + L::oB;
+  int32_t* const base = reinterpret_cast<int32_t*>(op_dyn) + L::oBase;
+  const int* const start = reinterpret_cast<const int*>(op_dyn) + L::oStart;
+  const int* const slot = reinterpret_cast<const int*>(op_dyn) + L::oSlot;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float* const qarg = op_dyn + L::oQueue + warp * 128;
+  int* const qslot = reinterpret_cast<int*>(qarg) + 64;
+  int nlev;
+  const bool mine = op_block_schedule(a.bb_inds, a.bb_data, op_dyn, nlev);
+  if (blockIdx.x == 0 && tid == 0) *taken = mine;
+  if (!mine) return;
+  const float sd0 = a.bb_data[0];
+  const int first = slot[0] * U * PS;  // step 0 fills the first date
+  const int bits = a.num_bits;
+  const uint32_t mask = bits >= 32 ? 0xffffffffu : (1u << bits) - 1u;
+  const float scale = ldexpf(1.0f, -bits);
+  const int nm = min(kOpModels, a.num_models - m0);
+  // block q holds the paths n = 32 q .. 32 q + 31 (of 1 .. num_mc_it)
+  const int64_t nblk = (int64_t)a.num_mc_it / 32 + 1;
+  const int64_t lo = nblk * blockIdx.x / gridDim.x, hi = nblk * (blockIdx.x + 1) / gridDim.x;
+  double acc[kOpModels];
+#pragma unroll
+  for (int mm = 0; mm < kOpModels; mm++) acc[mm] = 0.0;
+  for (int k = tid; k < K; k += kBlkThreads) base[k] = 0;
+  uint32_t gray = 0;  // the Gray code whose directions base holds
+  for (int64_t q = lo; q < hi; q++) {
+    const uint32_t n0 = (uint32_t)(32 * q), g0 = ((n0 >> 1) ^ n0) & mask;
+    for (int k = tid; k < K; k += kBlkThreads) {
+      int32_t x = base[k];
+      for (uint32_t f = g0 ^ gray; f != 0u; f &= f - 1u) x ^= dirT[(int64_t)(__ffs((int)f) - 1) * K + k];
+      base[k] = x;
+    }
+    gray = g0;
+    __syncthreads();
+    // -- Gaussians (:120-136) of the Sobol points (:13-33) --
+    int nq = 0;  // queued tail arguments
+    auto flush = [&](int n) {
+      __syncwarp();
+      float g = 0.0f;
+      int to = 0;
+      if (lane < n) {
+        g = gauss_tail(qarg[lane]);
+        to = qslot[lane];
+      }
+      const float more = qarg[32 + lane];
+      const int more_to = qslot[32 + lane];
+      if (lane < n) B_[to] = g;
+      __syncwarp();
+      qarg[lane] = more;
+      qslot[lane] = more_to;
+      __syncwarp();
+    };
+    constexpr int kGroups = (K + 31) / 32, kParts = 32 / kBlkRuns;
+    for (int it = warp; it < kGroups * kParts; it += kBlkWarps) {
+      const int k = (it / kParts) * 32 + lane, r0 = (it % kParts) * kBlkRuns;
+      const bool on = k < K;
+      const int kk = on ? k : K - 1;
+      const int to = (slot[kk / U] * U + kk % U) * PS + r0;
+      int32_t v[5];
+#pragma unroll
+      for (int c = 0; c < 5; c++) v[c] = c < bits ? dirT[(int64_t)c * K + kk] : 0;
+      int32_t x = base[kk];
+      const int rg = r0 ^ (r0 >> 1);  // bits 2 .. 4
+#pragma unroll
+      for (int c = 2; c < 5; c++)
+        if ((rg >> c) & 1) x ^= v[c];
+#pragma unroll
+      for (int t = 0; t < kBlkRuns; t++) {
+        if (t > 0) x ^= v[(t & 1) ? 0 : (t & 2) ? 1 : 2];
+        const float dp = (float)x * scale - 0.5f;
+        const bool tail = on && !gauss_is_central(dp);
+        const float g = gauss_central(dp);
+        if (on && !tail) B_[to + t] = g;
+        const unsigned ball = __ballot_sync(kAll, tail);
+        if (tail) {
+          const int at = nq + __popc(ball & ((1u << lane) - 1u));
+          qarg[at] = dp;
+          qslot[at] = to + t;
+        }
+        nq += __popc(ball);
+        if (nq >= 32) {
+          flush(32);
+          nq -= 32;
+        }
+      }
+    }
+    flush(nq);
+    __syncthreads();
+    // -- bridge (:142-165) in place, a level at a time --
+    if (warp < U) B_[first + warp * PS + lane] = sd0 * B_[first + warp * PS + lane];
+    __syncthreads();
+    for (int v = 1; v <= nlev; v++) {
+      const int s0 = start[v], cnt = (start[v + 1] - s0) * U;
+      for (int e = warp; e < cnt; e += kBlkWarps) {
+        const int at = s0 + e / U, u = (e % U) * PS + lane;
+        const float4 w4 = *reinterpret_cast<const float4*>(op_dyn + L::oStep + 4 * at);
+        const float2 w2 = *reinterpret_cast<const float2*>(op_dyn + L::oStep2 + 2 * at);
+        const int l = __float_as_int(w4.x), kk = __float_as_int(w4.y), j = __float_as_int(w4.z);
+        float val = w2.x * B_[kk + u] + w4.w * B_[l + u];
+        if (j >= 0) val = val + w2.y * B_[j + u];
+        B_[l + u] = val;
+      }
+      __syncthreads();
+    }
+    // -- per model: exponentials (:188-215), prices and payoff (:216-292) --
+    const int64_t n = 32 * q + lane;
+    const bool path = n >= 1 && n <= a.num_mc_it;
+#pragma unroll
+    for (int mm = 0; mm < kOpModels; mm++) {
+      if (mm >= nm) break;
+      const int m = m0 + mm;
+      const float* vol = a.md_vols + (int64_t)m * K;
+      const float* dr = a.md_drifts + (int64_t)m * K;
+      const float* st = a.md_sts + (int64_t)m * U;
+      float cm[U][U];
+#pragma unroll
+      for (int u = 0; u < U; u++)
+#pragma unroll
+        for (int i = 0; i <= u; i++) cm[u][i] = a.md_cs[((int64_t)m * U + u) * U + i];
+      float sc[U], price[U];
+      bool hit = false;
+#pragma unroll
+      for (int u = 0; u < U; u++) sc[u] = 1.0f;
+      constexpr int kChunks = (D + kBlkDates - 1) / kBlkDates;
+      for (int c = 0; c <= kChunks; c++) {
+        if (warp < kBlkWarps - 1) {
+          float* const E = op_dyn + L::oE + (c & 1) * kBlkDates * U * 32;
+          const int d1 = min(D, (c + 1) * kBlkDates);
+          for (int d = c * kBlkDates + warp; d < d1; d += kBlkWarps - 1) {
+            float inc[U];  // differences of consecutive dates (:167-175)
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+              const float b = B_[(d * U + u) * PS + lane];
+              inc[u] = d > 0 ? b - B_[((d - 1) * U + u) * PS + lane] : b;
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+              float noise = 0.0f;
+#pragma unroll
+              for (int i = 0; i <= u; i++) noise = noise + inc[i] * cm[u][i];
+              E[((d - c * kBlkDates) * U + u) * 32 + lane] = f32exp(dr[d * U + u] + noise * vol[d * U + u]);
+            }
+          }
+        } else if (c > 0) {
+          const float* const E = op_dyn + L::oE + ((c - 1) & 1) * kBlkDates * U * 32;
+          const float s0 = st[0], s1 = st[1], s2 = st[2];
+          const int nd = min(kBlkDates, D - (c - 1) * kBlkDates);
+#pragma unroll 4
+          for (int d = 0; d < nd; d++) {
+#pragma unroll
+            for (int u = 0; u < U; u++) sc[u] = sc[u] * E[(d * U + u) * 32 + lane];
+            price[0] = s0 * sc[0];
+            price[1] = s1 * sc[1];
+            price[2] = s2 * sc[2];
+            hit = hit || (price[0] <= 2630.6349999999998f || price[1] <= 8288.0f || price[2] <= 840.0f);
+          }
+        }
+        __syncthreads();
+      }
+      if (warp == kBlkWarps - 1 && path) {
+        const float* disc = a.md_discts + (int64_t)m * a.num_discts;
+        const float price1 = 100.0f * disc[0];
+        const bool goto40 = hit && (price[0] < 3758.05f || price[1] < 11840.0f || price[2] < 1200.0f);
+        const float amt = goto40 ? 1000.0f * fmin_payoff(price) : 1000.0f;
+        const float pay = price1 + amt * disc[1];
+        acc[mm] += (double)pay;
+        if (a.pay_out) a.pay_out[(n - 1) * a.num_models + m] = pay;
+      }
+    }
+  }
+  if (warp == kBlkWarps - 1) {
+#pragma unroll
+    for (int mm = 0; mm < kOpModels; mm++) {  // the CTA's sum, in a fixed order
+      if (mm >= nm) break;
+      double sum = acc[mm];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(kAll, sum, o);
+      double* const out = partial + (int64_t)mm * slots;
+      for (int b = blockIdx.x + lane * gridDim.x; b < slots; b += 32 * gridDim.x) out[b] = lane == 0 && b == blockIdx.x ? sum : 0.0;
+    }
   }
 }
 
@@ -810,6 +1109,8 @@ __global__ void __launch_bounds__(kSeqThreads) op_seq_reduce_kernel(const float*
 }
 
 constexpr size_t kWarpSmem3 = sizeof(float) * OpWarpSmem<3>::kWords;
+constexpr size_t kBlkSmem = sizeof(float) * OpBlk::kWords;
+static_assert(kBlkSmem <= 227 * 1024, "one CTA per SM");
 
 // CTAs of the paths kernel for `paths` paths of contract c: eight 128-thread
 // CTAs per SM (thread per path), or two 7-warp CTAs per SM (warp per path,
@@ -887,6 +1188,9 @@ int op_launch(futhark_context* ctx, const op_args* q, float* out, void* scratch)
   if (priced && c == 3) {
     cudaError_t e = cudaFuncSetAttribute((const void*)op_paths_warp_kernel<3>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWarpSmem3);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute((const void*)op_paths_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kBlkSmem);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "option pricing attributes");
     const int64_t kb = (int64_t)q->num_dates * q->num_und * q->num_bits;
     op_transpose_dirs_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((kb + 255) / 256, 1024)), 256, 0,
@@ -897,10 +1201,19 @@ int op_launch(futhark_context* ctx, const op_args* q, float* out, void* scratch)
   for (int m0 = 0; m0 < q->num_models; m0 += kOpModels) {
     const int nm = std::min(kOpModels, q->num_models - m0);
     if (priced) {
+      cudaError_t e_;
       if (c == 1) op_paths_kernel<1><<<(unsigned)T, kOpThreads, 0, ctx->stream>>>(a, m0, partial);
       else if (c == 2) op_paths_kernel<2><<<(unsigned)T, kOpThreads, 0, ctx->stream>>>(a, m0, partial);
-      else
-        op_paths_warp_kernel<3><<<(unsigned)T, kWarpPathWarps * 32, kWarpSmem3, ctx->stream>>>(a, dirT, m0, partial);
+      else {
+        // where the partial sums end: contract 3 has at most two of eight CTAs per SM
+        int* taken = reinterpret_cast<int*>(static_cast<char*>(scratch) + partial_bytes(ctx) - 256);
+        const int64_t nblk = (int64_t)q->num_mc_it / 32 + 1;
+        op_paths_block_kernel<<<(unsigned)std::min<int64_t>(ctx->num_sms, std::min(T, nblk)), kBlkThreads, kBlkSmem,
+                                ctx->stream>>>(a, dirT, m0, partial, (int)T, taken);
+        if ((e_ = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e_, "option pricing launch");
+        op_paths_warp_kernel<3><<<(unsigned)T, kWarpPathWarps * 32, kWarpSmem3, ctx->stream>>>(a, dirT, m0, partial,
+                                                                                              taken);
+      }
       const cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return cuda_fail(ctx, e, "option pricing launch");
     }
