@@ -374,9 +374,26 @@ __device__ __forceinline__ void col_stage_chunk(const TkeArgs& p, float* st, int
   }
 }
 
+// The same where every column is a run of whole 16-byte chunks (VEC): lane l copies
+// its own column's chunk of each field into st[field][column][z], one copy each,
+// and alone reads it back, four z per access.
+__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void col_stage_vec(const TkeArgs& p, float* st, int64_t col, int k, int lane) {
+  const int64_t g = col * p.Z + k * kColCh;
+  float* d = st + lane * kColCh;
+  cp_async16(d, p.tketau + g);
+  cp_async16(d + 32 * kColCh, p.kappaM + g);
+  cp_async16(d + 2 * 32 * kColCh, p.mxl + g);
+  cp_async16(d + 3 * 32 * kColCh, p.forc + g);
+}
+
 // Chunk k of tketaup1 -- what a cell keeps where the solution does not apply
 // -- into st[z - k*kColCh][column], in the pattern of col_stage_chunk.
 constexpr int kColUpdFloats = kColCh * kColPad;
+static_assert(4 * 32 * kColCh <= kColStageFloats && kColStageFloats % 4 == 0 && kColWarpFloats % 4 == 0, "VEC stages");
 static_assert(2 * kColUpdFloats <= kColStages * kColStageFloats, "update stages reuse the forward stages");
 __device__ __forceinline__ void col_stage_update(const TkeArgs& p, float* st, int64_t col0, int64_t ncol, int k,
                                                  int lane) {
@@ -397,8 +414,14 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // At most 128 registers (four CTAs' worth per SM): two CTAs then leave room
 // for two advection CTAs beside them.
+// VEC: zdim is a multiple of 4 and the six fields start on 16-byte boundaries.  A
+// lane then moves its own column four z at a time -- the staged fields, tketaup1 and
+// the result as they lie in memory, the quotients as [chunk][column][8] -- and no
+// tile turns lanes between z and columns: 100 levels take 41 us with an SM to
+// themselves, 57 the other way, and 200 x 200 of them 70 against 86.
+template <bool VEC>
 __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p) {
-  extern __shared__ float smem[];
+  extern __shared__ __align__(16) float smem[];
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t ncol = (int64_t)p.X * p.Y;
@@ -418,6 +441,30 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
   const int64_t qs = p.ncolp;
   float* q0 = p.q0 + col;
   float* q1 = p.q1 + col;
+  float* qv = p.q0 + 8 * col;  // VEC: chunk k's quotients at 8 qs k
+  auto put_quotients = [&](int z, float v0, float v1) {
+    if constexpr (VEC) {
+      float* o = qv + (int64_t)(z / kColCh) * 8 * qs + z % kColCh;
+      o[0] = v0;
+      o[kColCh] = v1;
+    } else {
+      const int64_t o = (int64_t)z * qs;
+      q0[o] = v0;
+      q1[o] = v1;
+    }
+  };
+  auto stage = [&](int k) {
+    float* const to = st + (k % kColStages) * kColStageFloats;
+    if constexpr (VEC) {
+      if (valid) col_stage_vec(p, to, col, k, lane);
+    } else {
+      col_stage_chunk(p, to, col0, ncol, k, lane);
+    }
+  };
+  // field f of this column at z of the chunk staged in buf
+  auto field = [&](const float* buf, int f, int zz) {
+    return VEC ? buf[(f * 32 + lane) * kColCh + zz] : buf[(f * kColCh + zz) * kColPad + lane];
+  };
 
   // Forward, staged a chunk of kColCh z at a time: (A) the coefficients
   // (tke.fut:103-210); (B) tridagPar's recurrences 1 (the 4-tuple scan for
@@ -428,9 +475,9 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
   // and its like, the coefficients of a chunk's z without a branch and ahead of
   // the recurrences, and once more one z at a time with exact division where an
   // interior column left their range.  (200 x 200 x 100 with sea floor at every
-  // depth: 130 -> 86 us for the kernel, which spent its time on the chain of each z,
+  // depth: 130 -> 70 us for the kernel, which spent its time on the chain of each z,
   // six divisions and their branches, at two warps per scheduler; what bounds it now
-  // is that chain and the instructions, half an issue slot per cycle.)
+  // is that chain.)
   auto forward = [&](auto near) -> bool {
     constexpr bool kNear = decltype(near)::value;
     RangeCheck in;
@@ -438,9 +485,9 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
     float dm = 0.0f, cprev = 0.0f;
     double rbpprev = 0.0;         // 1 / b' of z - 1 (DR_)
     float bprev = 1.0f, rbprev = 1.0f;  // b' of z - 1 and its reciprocal (near_div)
-    col_stage_chunk(p, st, col0, ncol, 0, lane);
+    stage(0);
     cp_async_commit();
-    if (nch > 1) col_stage_chunk(p, st + kColStageFloats, col0, ncol, 1, lane);
+    if (nch > 1) stage(1);
     cp_async_commit();
     // the per-z constants of the next chunk, loaded a chunk ahead: lane l
     // holds dzw and dzt of z + 1 for z = (chunk) * kColCh + l % kColCh
@@ -452,7 +499,7 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
     };
     ld_consts(0);
     for (int k = 0; k < nch; k++) {
-      if (k + 2 < nch) col_stage_chunk(p, st + ((k + 2) % kColStages) * kColStageFloats, col0, ncol, k + 2, lane);
+      if (k + 2 < nch) stage(k + 2);
       cp_async_commit();
       cp_async_wait_all_but_one();  // chunks k and k + 1 have landed
       __syncwarp();
@@ -471,6 +518,30 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
         // (A) for the chunk's four z, independent of one another and of (B);
         // selections instead of branches
         float a_[kColCh], b_[kColCh], c_[kColCh], d_[kColCh];
+        float ft[kColCh], fk[kColCh + 1], fm[kColCh], ff[kColCh];
+        if constexpr (VEC) {
+          auto ld4 = [&](int f, float* v) {
+            const float4 t = *reinterpret_cast<const float4*>(cur + (f * 32 + lane) * kColCh);
+            v[0] = t.x;
+            v[1] = t.y;
+            v[2] = t.z;
+            v[3] = t.w;
+          };
+          ld4(0, ft);
+          ld4(1, fk);
+          ld4(2, fm);
+          ld4(3, ff);
+        } else {
+#pragma unroll
+          for (int zz = 0; zz < kColCh; zz++) {
+            ft[zz] = field(cur, 0, zz);
+            fk[zz] = field(cur, 1, zz);
+            fm[zz] = field(cur, 2, zz);
+            ff[zz] = field(cur, 3, zz);
+          }
+        }
+        fk[kColCh] = field(nxt, 1, 0);
+        float v0[kColCh], v1[kColCh];
 #pragma unroll
         for (int zz = 0; zz < kColCh; zz++) {
           const int z = zbase + zz;
@@ -478,13 +549,10 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
           const float fac = __shfl_sync(kAll, fac_l, zz);
           const float dz = __shfl_sync(kAll, dz_l, zz), rdz = __shfl_sync(kAll, rdz_l, zz);
           const float dd = top ? M_(0.5f, dz) : dz, rdd = top ? M_(2.0f, rdz) : rdz;
-          const float t = cur[zz * kColPad + lane];
-          const float kap = cur[(kColCh + zz) * kColPad + lane];
-          const float fo = cur[(3 * kColCh + zz) * kColPad + lane];
-          const float kapn = zz + 1 < kColCh ? cur[(kColCh + zz + 1) * kColPad + lane] : nxt[kColCh * kColPad + lane];
-          const float d0 = z < Z - 1 ? M_(fac, A_(kap, kapn)) : 0.0f;  // delta (:103-108)
+          const float t = ft[zz], fo = ff[zz];
+          const float d0 = z < Z - 1 ? M_(fac, A_(fk[zz], fk[zz + 1])) : 0.0f;  // delta (:103-108)
           const bool edge = land && z == ks, water = land && z >= ks;
-          const float mx = water ? cur[(2 * kColCh + zz) * kColPad + lane] : 1.0f;
+          const float mx = water ? fm[zz] : 1.0f;
           const float t0 = max_(0.0f, t), sq = near_sqrt(t0);
           a_[zz] = !edge && water && z > 0 ? near_div(-dm, dd, rdd) : 0.0f;
           // 1 + (delta of the levels around) / dz + dissipation: the edge has
@@ -497,9 +565,9 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
           c_[zz] = z < Z - 1 && water ? near_div(-d0, dz, rdz) : 0.0f;
           const float tmp = A_(t, M_(kDtTke, fo));
           d_[zz] = water ? tmp : 0.0f;
-          if (top && water) d_[zz] = A_(tmp, D_(M_(kDtTke, fts), M_(0.5f, dz)));
+          if ((!VEC || zz == kColCh - 1) && top && water) d_[zz] = A_(tmp, D_(M_(kDtTke, fts), M_(0.5f, dz)));
           dm = d0;
-          if (zz < zn) {
+          if (VEC || zz < zn) {
             in.divisor(mx);
             in.dividend(t0);
             in.dividend(d0);
@@ -508,7 +576,7 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
         // (B), (C)
 #pragma unroll
         for (int zz = 0; zz < kColCh; zz++) {
-          if (zz >= zn) break;
+          if (!VEC && zz >= zn) break;
           float bp, yp;
           if (zz == 0 && k == 0) {  // the neutral elements
             b0 = b_[0];
@@ -542,11 +610,14 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
           cprev = c_[zz];
           bprev = bp;
           rbprev = rb;
-          if (inner) {
-            const int64_t o = (int64_t)(zbase + zz) * qs;
-            q0[o] = yp == 0.0f ? M_(yp, rb) : near_div(yp, bp, rb);
-            q1[o] = S_(0.0f, near_div(cprev, bp, rb));
-          }
+          v0[zz] = yp == 0.0f ? M_(yp, rb) : near_div(yp, bp, rb);
+          v1[zz] = S_(0.0f, near_div(cprev, bp, rb));
+          if (!VEC && inner) put_quotients(zbase + zz, v0[zz], v1[zz]);
+        }
+        if (VEC && inner) {
+          float4* o = reinterpret_cast<float4*>(qv + (int64_t)k * 8 * qs);
+          o[0] = make_float4(v0[0], v0[1], v0[2], v0[3]);
+          o[1] = make_float4(v1[0], v1[1], v1[2], v1[3]);
         }
       } else {
         const double rdz_l = Rd_(dz_l);  // the quotients by dz of the interior levels (DR_)
@@ -557,11 +628,11 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
         const float dz = __shfl_sync(kAll, dz_l, zz);
         const double rdz = __shfl_sync(kAll, rdz_l, zz);
         const int z = zbase + zz;
-        const float t = cur[zz * kColPad + lane];
-        const float kap = cur[(kColCh + zz) * kColPad + lane];
-        const float mx = cur[(2 * kColCh + zz) * kColPad + lane];
-        const float fo = cur[(3 * kColCh + zz) * kColPad + lane];
-        const float kapn = zz + 1 < kColCh ? cur[(kColCh + zz + 1) * kColPad + lane] : nxt[kColCh * kColPad + lane];
+        const float t = field(cur, 0, zz);
+        const float kap = field(cur, 1, zz);
+        const float mx = field(cur, 2, zz);
+        const float fo = field(cur, 3, zz);
+        const float kapn = zz + 1 < kColCh ? field(cur, 1, zz + 1) : field(nxt, 1, 0);
         const float d0 = z < Z - 1 ? M_(fac, A_(kap, kapn)) : 0.0f;  // delta (:103-108)
         const bool edge = land && z == ks, water = land && z >= ks;
         const float sq = __fsqrt_rn(max_(0.0f, t));
@@ -613,11 +684,7 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
         const float ypz = A_(r0, M_(r1, y0));
         cprev = c_;
         rbpprev = rbp;
-        if (inner) {
-          const int64_t o = (int64_t)z * qs;
-          q0[o] = DR_(ypz, rbp);
-          q1[o] = S_(0.0f, DR_(c_, rbp));
-        }
+        if (inner) put_quotients(z, DR_(ypz, rbp), S_(0.0f, DR_(c_, rbp)));
       }
       }
       __syncwarp();  // the next iteration refills this chunk's stage
@@ -636,11 +703,66 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
   // of the chunk after next (registers) and tketaup1 three chunks on
   // (cp.async) load meanwhile: a backward chunk is little work, so one chunk
   // ahead left the loads' latency exposed.
-  float* ust = st;
-  const float yn = inner ? q0[(int64_t)(Z - 1) * qs] : 0.0f;  // y'_{n-1} / b'_{n-1}
   r0 = 0.0f;
   r1 = 1.0f;
   if (valid && !inner) p.tke_surf_corr_out[col] = 0.0f;
+  // the top cell's correction, clip and lateral diffusion (:219-263)
+  auto top_cell = [&](float v) {
+    const int z = Z - 1;
+    float tp = (land && z >= ks) ? v : p.tketaup1[col * Z + z];
+    p.tke_surf_corr_out[col] = tp < 0.0f ? D_(M_(M_(-tp, 0.5f), p.dzw[z]), kDtTke) : 0.0f;
+    tp = tp < 0.0f ? 0.0f : tp;
+    return A_(tp, M_(M_(kDtTke, p.maskW[col * Z + z]),
+                     A_(D_(S_(diff_east(p, x, y, z), diff_east(p, x - 1, y, z)), M_(p.cost[y], p.dxt[x])),
+                        D_(S_(diff_north(p, x, y, z), diff_north(p, x, y - 1, z)), M_(p.cost[y], p.dyt[y])))));
+  };
+  if constexpr (VEC) {
+    if (!valid) return;
+    // quotients and tketaup1 of chunks k (Q[0]), k - 1 and k - 2
+    struct Chunk {
+      float4 a, b, t;
+    };
+    const float4* tp = reinterpret_cast<const float4*>(p.tketaup1 + col * Z);
+    float4* op = reinterpret_cast<float4*>(p.tketaup1_out + col * Z);
+    auto load = [&](int k) {
+      Chunk c{make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+      if (k >= 0) {
+        c.t = tp[k];
+        if (inner) {
+          const float4* q = reinterpret_cast<const float4*>(qv + (int64_t)k * 8 * qs);
+          c.a = q[0];
+          c.b = q[1];
+        }
+      }
+      return c;
+    };
+    Chunk c0 = load(nch - 1), c1 = load(nch - 2);
+    const float yn = c0.a.w;  // y'_{n-1} / b'_{n-1}; that element folds the neutral (0, 1)
+    c0.a.w = 0.0f;
+    c0.b.w = 1.0f;
+    for (int k = nch - 1; k >= 0; k--) {
+      const Chunk c2 = load(k - 2);
+      float v[kColCh], vtop = 0.0f;
+      const float qa0[kColCh] = {c0.a.x, c0.a.y, c0.a.z, c0.a.w}, qa1[kColCh] = {c0.b.x, c0.b.y, c0.b.z, c0.b.w};
+      const float u[kColCh] = {c0.t.x, c0.t.y, c0.t.z, c0.t.w};
+#pragma unroll
+      for (int zz = kColCh - 1; zz >= 0; zz--) {
+        r0 = A_(qa0[zz], M_(qa1[zz], r0));
+        r1 = M_(r1, qa1[zz]);
+        const int z = k * kColCh + zz;
+        const float sol = A_(r0, M_(r1, yn));
+        if (zz == kColCh - 1) vtop = sol;
+        v[zz] = inner && land && z >= ks ? sol : u[zz];
+      }
+      if (k == nch - 1 && inner) v[kColCh - 1] = top_cell(vtop);
+      op[k] = make_float4(v[0], v[1], v[2], v[3]);
+      c0 = c1;
+      c1 = c2;
+    }
+    return;
+  } else {
+  float* ust = st;
+  const float yn = inner ? q0[(int64_t)(Z - 1) * qs] : 0.0f;  // y'_{n-1} / b'_{n-1}
   // quotients of chunk k (qa), k - 1 (qb) and k - 2 (loaded this iteration)
   // in registers; tketaup1 of chunks k .. k - kUpd + 1 in flight (cp.async)
   constexpr int kUpd = 4;
@@ -684,14 +806,7 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
         r0 = rn0;
         r1 = rn1;
         float v = A_(r0, M_(r1, yn));
-        if (z == Z - 1) {  // the top cell
-          float tp = (land && z >= ks) ? v : p.tketaup1[col * Z + z];
-          p.tke_surf_corr_out[col] = tp < 0.0f ? D_(M_(M_(-tp, 0.5f), p.dzw[Z - 1]), kDtTke) : 0.0f;
-          tp = tp < 0.0f ? 0.0f : tp;
-          v = A_(tp, M_(M_(kDtTke, p.maskW[col * Z + z]),
-                        A_(D_(S_(diff_east(p, x, y, z), diff_east(p, x - 1, y, z)), M_(p.cost[y], p.dxt[x])),
-                           D_(S_(diff_north(p, x, y, z), diff_north(p, x, y - 1, z)), M_(p.cost[y], p.dyt[y])))));
-        }
+        if (z == Z - 1) v = top_cell(v);
         tile[zz * kColPad + lane] = v;
       }
     }
@@ -717,6 +832,7 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
       qb0[zz] = qc0[zz];
       qb1[zz] = qc1[zz];
     }
+  }
   }
 }
 
@@ -814,13 +930,20 @@ int step_launch(futhark_context* ctx, const tke_step_args* q) {
   // the columns: coefficients, tridagPar, tketaup1 (tke.fut:103-263)
   const int64_t col_blocks = (X * Y + 32 * kColWarps - 1) / (32 * kColWarps);
   if (col_blocks > INT32_MAX) return set_error(ctx, FUTHARK_PROGRAM_ERROR, "tke step: too many columns");
+  const auto vec16 = [](const void* f) { return ((uintptr_t)f & 15) == 0; };
+  const bool vec = Z % kColCh == 0 && vec16(p.tketau) && vec16(p.kappaM) && vec16(p.mxl) && vec16(p.forc) &&
+                   vec16(p.tketaup1) && vec16(p.tketaup1_out);
+  const auto column = vec ? tke_column_kernel<true> : tke_column_kernel<false>;
   if (!ctx->smem_raised) {  // once per context: host time the step need not spend
-    e = cudaFuncSetAttribute((const void*)tke_column_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute((const void*)tke_column_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kColSmem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute((const void*)tke_column_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kColSmem);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "tke column attributes");
     ctx->smem_raised = true;
   }
-  tke_column_kernel<<<(unsigned)col_blocks, 32 * kColWarps, kColSmem, s>>>(p);
+  column<<<(unsigned)col_blocks, 32 * kColWarps, kColSmem, s>>>(p);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(ctx, e, "tke column launch");
   // advection and dtketau: (y, z) tiles of at most 31 owned levels plus a
