@@ -29,7 +29,7 @@ ORACLE_DIR = os.path.join(REPO, "oracle")
 ORACLE_LIB = os.path.join(ORACLE_DIR, "liblvc_oracle.so")
 
 SOURCES = ["lvc_runtime.cu"]
-HEADERS = ["lvc_kernels.cuh", "lvc_layout.h", "lvc_probe.cuh", "lvc_line.cuh", "lvc_pair.cuh", "lvc_tridiag.cuh",
+HEADERS = ["lvc_kernels.cuh", "lvc_layout.h", "lvc_probe.cuh", "lvc_line.cuh", "lvc_pair.cuh", "lvc_tall.cuh", "lvc_tridiag.cuh",
            "exact_math.cuh"]
 TKE_SOURCES = ["tke_runtime.cu"]
 TKE_HEADERS = ["exact_math.cuh", "fut_api.cuh"]

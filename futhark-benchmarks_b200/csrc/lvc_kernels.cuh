@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(256) lvc_setup_kernel(const CalibDev* __restri
                                                         double* __restrict__ tabs) {
   const CalibDev c = calibs[blockIdx.x];
   const int X = c.Xr, Y = c.Yr, T = c.numT, Xp = c.Xp;
-  const bool line = c.kind == kKindLine;
+  const bool line = c.kind != kKindChunk;
   const TabLayout L = tab_layout(c.numX, c.numY, T, Xp, c.kind);
   double* tab = tabs + c.tab;
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -164,7 +164,7 @@ __device__ __forceinline__ int find_calib(const int64_t* __restrict__ start, int
 __device__ __forceinline__ void y_pivots(const CalibDev& c, int k0, double* __restrict__ tabs, double (*co)[4]) {
   const int lane = threadIdx.x & 31;
   const int Y = c.numY, steps = c.numT - 1;  // a padding row's coefficients are zero: b' = dt, no multipliers
-  const bool line = c.kind == kKindLine;
+  const bool line = c.kind != kKindChunk;
   const TabLayout L = tab_layout(c.numX, Y, c.numT, c.Xp, c.kind);
   double* tab = tabs + c.tab;
   const int k = k0 + lane;
@@ -258,7 +258,7 @@ __device__ __forceinline__ void x_pivots(const CalibDev& c, int64_t r0, double* 
                                          PV* __restrict__ piv, double (*co)[4], double (*tile)[kPivotCols + 1]) {
   const int lane = threadIdx.x & 31;
   const int X = c.Xr, Y = c.numY;
-  const bool line = c.kind == kKindLine;
+  const bool line = c.kind != kKindChunk;
   const TabLayout L = tab_layout(c.numX, Y, c.numT, c.Xp, c.kind);
   double* tab = tabs + c.tab;
   const int64_t rows = (int64_t)(c.numT - 1) * Y;
@@ -296,7 +296,10 @@ __device__ __forceinline__ void x_pivots(const CalibDev& c, int64_t r0, double* 
                        : 0.0;
   if (lane < nr) tab[line ? L.stab + ((int64_t)k * Y + j) * 8 + kSlotE : L.eyt + (int64_t)k * L.eyt_ld + j] = e;
   double rb = 0.0, c_prev = 0.0;  // 1/b' and c of the column before: zero before the first
-  for (int c0 = 0; c0 < LD; c0 += kPivotCols) {
+  const bool tall = c.kind == kKindTall;  // r0 is then a row group's first row
+  PV* const group = piv + c.piv + tall_piv(c.numX, Y, k, j & ~31, 0);
+  const int width = tall ? c.numX : LD;
+  for (int c0 = 0; c0 < width; c0 += kPivotCols) {
     __syncwarp();
     co[lane][0] = v0;
     co[lane][1] = v1;
@@ -324,6 +327,15 @@ __device__ __forceinline__ void x_pivots(const CalibDev& c, int64_t r0, double* 
       tile[lane][m] = rb;
     }
     for (int m = max(n, 0); m < kPivotCols; m++) tile[lane][m] = 0.0;  // padding columns
+    if (tall) {  // a pair of columns of the 32 rows at a time
+#pragma unroll 4
+      for (int m = 0; m < kPivotCols; m += 2) {
+        PV* o = group + (int64_t)(c0 + m) * 32 + 2 * lane;
+        o[0] = (PV)tile[lane][m];
+        o[1] = (PV)tile[lane][m + 1];
+      }
+      continue;
+    }
     __syncwarp();
     const bool w = c0 + lane < LD;
     auto put = [&](int q) {

@@ -27,6 +27,7 @@ constexpr int kLineK = 16;       // line-kernel chunk: elements of a line per la
 enum : int32_t {
   kKindChunk = 0,  // lanes own 8/16-element chunks of a row (any numX <= 512, HBM-state capable)
   kKindLine = 1,   // lanes own whole lines of the grid (numX <= 256, on chip)
+  kKindTall = 2,   // paired line kernel with its pivots in tensor memory: twice the rows per CTA
 };
 
 // One calibration, as the device sees it.  Filled by the host runtime.
@@ -115,6 +116,11 @@ enum : int {
 // aligned) for the paired kernel.
 LVC_HD int line_ld(int X) { return X | 1; }
 LVC_HD int pair_ld(int X) { return X + 2; }
+// Tall kernel: the pivots as its threads load them, a lane per row of a group of 32
+// rows and a pair of columns at a time: element (row j, column i) of step k.
+LVC_HD int64_t tall_piv(int X, int Y, int k, int j, int i) {
+  return (((int64_t)k * (Y / 32) + j / 32) * (X / 2) + i / 2) * 64 + (j % 32) * 2 + (i & 1);
+}
 LVC_HD int64_t round4(int64_t n) { return (n + 3) & ~int64_t(3); }
 
 // Elements of the X-direction pivot array of one calibration (plus 4 of

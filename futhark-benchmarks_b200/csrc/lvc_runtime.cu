@@ -35,6 +35,7 @@
 #include "lvc_kernels.cuh"
 #include "lvc_line.cuh"
 #include "lvc_pair.cuh"
+#include "lvc_tall.cuh"
 #include "lvc_tridiag.cuh"
 #include "tridiag.h"
 #include "lvc_probe.cuh"
@@ -412,6 +413,12 @@ using RbFn = void (*)(RollbackArgs<S, PV>);
 template <typename S, typename PV>
 RbFn<S, PV> rollback_fn(int kind, int NT, int KX, bool gs, bool full = false, bool pair = false,
                         int upw = 2) {
+  if (kind == kKindTall) {
+    if constexpr (std::is_same<S, double>::value && std::is_same<PV, double>::value) {
+      return lvc_line_tall_kernel;
+    }
+    return nullptr;
+  }
   if (kind == kKindLine && pair && upw == 1) {
     if (NT == 64) return lvc_line_pair_kernel<S, PV, 64, 1>;
     if (NT == 128) return lvc_line_pair_kernel<S, PV, 128, 1>;
@@ -508,6 +515,31 @@ bool line_pair_cfg(int X, int Y, int C, int max_smem, Config& cf, int upw = 2) {
   cf.upw = upw;
   cf.ld = pair_ld(Xt);
   cf.NT = 32 * NW;
+  cf.KX = kLineK;
+  cf.C = C;
+  cf.gstate = false;
+  cf.Ycs = Ycs;
+  cf.smem_bytes = (size_t)F.total;
+  cf.grid_elems = 0;
+  return true;
+}
+
+// Tall paired kernel (f64): the grid padded to 64, 128 or 256 columns and to C CTAs
+// of the 16384 cells that its 8 warps take.
+template <typename S>
+bool line_tall_cfg(int X, int Y, int max_smem, Config& cf) {
+  const int Xt = ceil_div(X, 64) * 64;
+  if (sizeof(S) != 8 || Xt > 256 || kTallWarps % (Xt / 32)) return false;
+  const int Ycs = kTallRounds * 32 * (kTallWarps / (Xt / 32));
+  const int C = ceil_div(Y, Ycs);
+  const TallLayout F = tall_layout(Xt, Ycs, C);
+  if (C > 8 || F.total > max_smem) return false;
+  cf.kind = kKindTall;
+  cf.full = false;
+  cf.pair = true;
+  cf.upw = 2;
+  cf.ld = pair_ld(Xt);
+  cf.NT = 32 * kTallWarps;
   cf.KX = kLineK;
   cf.C = C;
   cf.gstate = false;
@@ -660,7 +692,7 @@ double pair_cost(const Config& cf, int X, int Y, int outer) {
 // 128 x 256 and 64 x 256 in the smallest clusters and 267 in ones of CTAs of 4096
 // cells).
 template <typename S>
-Config default_config(int X, int Y, int max_smem, int outer = 0) {
+Config default_paired(int X, int Y, int max_smem, int outer) {
   if (outer <= 0 && whole_tiles(X, Y)) return unpadded_config<S>(X, Y, max_smem);
   Config best;
   double best_cost = 0.0;
@@ -674,6 +706,38 @@ Config default_config(int X, int Y, int max_smem, int outer = 0) {
   return best_cost > 0.0 ? best : unpadded_config<S>(X, Y, max_smem);
 }
 
+// What a time step costs, in microseconds, where a CTA of 8 warps has an SM to
+// itself -- the tall kernel and the paired one of two units per warp -- from the
+// clusters that fit on the chip at once and a step's time in each (the figures
+// stand at the tall kernel); many strikes (outer <= 0): per strike.
+double waves_cost(const Config& cf, int outer) {
+  static const double tall[] = {12.0, 14.1, 15.5, 15.5}, pair[] = {5.6, 7.2, 7.4, 7.7};
+  const int l = cf.C > 4 ? 3 : cf.C > 2 ? 2 : cf.C - 1;
+  const double step = cf.kind == kKindTall ? tall[l] : pair[l];
+  // clusters of more than two lie in one of the chip's eight GPCs of 18 or 16 SMs
+  const int slots = cf.C <= 2 ? 148 / cf.C : cf.C == 8 ? 15 : 8 * (16 / cf.C);
+  return outer <= 0 ? step / slots : step * ceil_div(outer, slots);
+}
+
+// The tall kernel takes over where the paired one needs a cluster and it is the
+// faster by 2 % (its step has been timed to a percent): 64 strikes of 256 x 256 30.7
+// us a step against 37.2, but 6 strikes 15.5 against 7.7.  In a batch it takes the
+// grids whose clusters of more than two it halves to two: other classes fill what
+// the paired kernel's clusters of eight leave idle, and the long steps end the batch
+// later (the 512-calibration mix: 253.3 ms without the tall kernel, 249.3 with
+// 128 x 256 and 256 x 128 in it, 262.0 with 256 x 256, 254.0 with 256 x 64, 128 x 128
+// and 64 x 256).
+template <typename S>
+Config default_config(int X, int Y, int max_smem, int outer = 0) {
+  const Config cf = default_paired<S>(X, Y, max_smem, outer);
+  Config tall;
+  if (cf.C == 1 || !line_tall_cfg<S>(X, Y, max_smem, tall)) return cf;
+  if (!cf.pair || (outer <= 0 && (cf.C <= 2 || tall.C > 2))) return cf;
+  const bool whole = cf.upw == 2 && cf.NT == 256;
+  const double cost = whole ? waves_cost(cf, outer) : pair_cost<S>(cf, X, Y, outer);
+  return waves_cost(tall, outer) < 0.98 * cost ? tall : cf;
+}
+
 // Every configuration that can run an X x Y grid: the search space of the
 // autotuner, in the order the built-in choice prefers them.  Splits thinner
 // than 16 rows per CTA (line family) or 8 (chunk family) are left out: the
@@ -683,6 +747,7 @@ std::vector<Config> enum_configs(int X, int Y, int max_smem) {
   std::vector<Config> v;
   Config cf;
   v = pair_configs<S>(X, Y, max_smem);
+  if (line_tall_cfg<S>(X, Y, max_smem, cf)) v.push_back(cf);
   for (int C = 1; C <= kMaxCluster; C *= 2) {
     if (line_full_cfg<S>(X, Y, C, max_smem, cf)) v.push_back(cf);
     if (line_generic_cfg<S>(X, Y, C, max_smem, cf) && (C == 1 || cf.Ycs >= 16)) v.push_back(cf);
@@ -696,6 +761,7 @@ std::vector<Config> enum_configs(int X, int Y, int max_smem) {
 
 int family_of(const Config& c) {
   if (c.kind == kKindChunk) return LVC_FAMILY_CHUNK;
+  if (c.kind == kKindTall) return LVC_FAMILY_LINE_TALL;
   if (c.pair) return c.upw == 1 ? LVC_FAMILY_LINE_PAIR1 : LVC_FAMILY_LINE_PAIR;
   return c.full ? LVC_FAMILY_LINE_FULL : LVC_FAMILY_LINE;
 }
@@ -1548,6 +1614,7 @@ int lvc_context_set_tuning_param(struct futhark_context* ctx, const char* param_
 namespace {
 
 const char* family_name(int fam, bool gstate) {
+  if (fam == LVC_FAMILY_LINE_TALL) return "line_tall";
   if (fam == LVC_FAMILY_LINE_PAIR1) return "line_pair1";
   if (fam == LVC_FAMILY_LINE_PAIR) return "line_pair";
   if (fam == LVC_FAMILY_LINE_FULL) return "line_full";
@@ -1908,13 +1975,14 @@ int lvc_tuning_load(struct futhark_context* ctx, const char* path) {
       lvc_shape sh{};
       sh.cluster = C;
       const std::string fs(fam);
-      sh.family = fs == "line_pair1"  ? LVC_FAMILY_LINE_PAIR1
+      sh.family = fs == "line_tall"   ? LVC_FAMILY_LINE_TALL
+                  : fs == "line_pair1" ? LVC_FAMILY_LINE_PAIR1
                   : fs == "line_pair" ? LVC_FAMILY_LINE_PAIR
                   : fs == "line_full" ? LVC_FAMILY_LINE_FULL
                   : fs == "line"      ? LVC_FAMILY_LINE
                                       : LVC_FAMILY_CHUNK;
       sh.hbm_state = fs == "chunk_hbm" ? 1 : 0;
-      const bool known = fs == "line_pair1" || fs == "line_pair" || fs == "line_full" || fs == "line" || fs == "chunk" || fs == "chunk_hbm";
+      const bool known = fs == "line_tall" || fs == "line_pair1" || fs == "line_pair" || fs == "line_full" || fs == "line" || fs == "chunk" || fs == "chunk_hbm";
       const int p = !strcmp(prec, "f64") ? LVC_F64 : !strcmp(prec, "f32state") ? LVC_F32_STATE : -1;
       if (!known || p < 0) rc = 1;
       else rc = lvc_tuning_set(ctx, X, Y, p, &sh);

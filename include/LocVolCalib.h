@@ -287,6 +287,7 @@ LVC_API int lvc_context_set_tuning_param(struct futhark_context *ctx, const char
 #define LVC_FAMILY_LINE_FULL 2 /* line family on full 32 x 32 tiles (numX, rows per CTA multiples of 32) */
 #define LVC_FAMILY_LINE_PAIR 3 /* full tiles walked two columns at a time (numX % 64 == 0) */
 #define LVC_FAMILY_LINE_PAIR1 4 /* the same with one unit per warp: twice the warps (numX % 32 == 0) */
+#define LVC_FAMILY_LINE_TALL 5 /* paired kernel, pivots in tensor memory: twice the rows per CTA (f64) */
 
 struct lvc_shape {
   int32_t family;       /* LVC_FAMILY_* */
@@ -340,7 +341,7 @@ LVC_API int lvc_autotune_plan(struct futhark_context *ctx, const struct lvc_cali
                               int32_t *streams, double *ms);
 /* The tuning parameters and the table as a tuning file of name=value lines:
  *   lvc.streams=4
- *   lvc.shape.f64.256x256=line_pair,8      (family: line_pair|line_pair1|line_full|line|chunk|chunk_hbm, cluster) */
+ *   lvc.shape.f64.256x256=line_pair,8      (family: line_tall|line_pair|line_pair1|line_full|line|chunk|chunk_hbm, cluster) */
 LVC_API int lvc_tuning_save(struct futhark_context *ctx, const char *path);
 LVC_API int lvc_tuning_load(struct futhark_context *ctx, const char *path);
 
