@@ -142,7 +142,7 @@ __device__ bool bridge_indices_valid(const int32_t* ind) {
 // (contract 2) a path's Gaussians come first, the central branch in every lane and
 // the tail arguments, 15 % of them, queued by the warp and evaluated 32 at a time: on
 // the fly nearly every Gaussian has some lane in its tail, with an f64 logarithm.
-// 1M paths 219 -> 137 us, 131072 45 -> 35, 16384 18.7 -> 14.6.  Contract 1 keeps the
+// 1M paths 219 -> 130 us, 131072 45 -> 32, 16384 18.7 -> 14.5.  Contract 1 keeps the
 // branch: its one Gaussian per path queued took 115 us for 8.4M paths against 108,
 // and with eight paths per lane at a time 103, but 50 against 36 for 2M.
 template <int C>
