@@ -1122,6 +1122,13 @@ int plan_new_locked(futhark_context* ctx, const lvc_calibration* cs, int n, int 
                                       : plan_build<float, float>(ctx, cs, n, P);
   if (rc) {
     plan_release(P);
+    // padded tables can be four times as large: without padding what fitted still does
+    // (a server's budget has decided on it beforehand)
+    if (rc == FUTHARK_OUT_OF_MEMORY && pad && max_sms == 0) {
+      cudaGetLastError();  // the failed allocation's
+      ctx->error.clear();
+      return plan_new_locked(ctx, cs, n, precision, out, pool, use_graph, max_sms, /*pad=*/false, alone);
+    }
     return rc;
   }
   *out = P;
