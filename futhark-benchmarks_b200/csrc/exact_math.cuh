@@ -43,19 +43,25 @@ __device__ __forceinline__ float near_sqrt(float x) {
 }
 
 // Whether the divisors seen so far lie inside (2^-40, 2^40) and the dividends are
-// zero or inside (2^-80, 2^80): in near_rcp's, near_div's and near_sqrt's range.  A NaN passes: the iterations return NaN for it, as division does.
+// zero or inside (2^-80, 2^80): in near_rcp's, near_div's and near_sqrt's range.
+// A NaN among them passes, and may: the iterations return NaN for it, as division
+// does.  But an infinite dividend makes a NaN where division gives an infinity, and
+// as a divisor or dividend further on that NaN would pass too, so every dividend is
+// to be seen here: by its quotient, where that is a divisor and bounds it, from
+// above at least (large).
 struct RangeCheck {
   float lo = 1.0f, hi = 1.0f, nlo = 1.0f, nhi = 1.0f;
   __device__ __forceinline__ void divisor(float x) {
     lo = fminf(lo, fabsf(x));
     hi = fmaxf(hi, fabsf(x));
   }
+  __device__ __forceinline__ void large(float x) { nhi = fmaxf(nhi, fabsf(x)); }
   __device__ __forceinline__ void dividend(float x) {
     nlo = fminf(nlo, x == 0.0f ? 1.0f : fabsf(x));
-    nhi = fmaxf(nhi, fabsf(x));
+    large(x);
   }
   // min_dividend: where quotients are dividends in turn
-  __device__ __forceinline__ bool ok(float min_dividend = 0x1p-80f) const { return lo > 0x1p-40f && hi < 0x1p40f && nlo > min_dividend && nhi < 0x1p80f; }
+  __device__ __forceinline__ bool ok(float min_dividend = 0x1p-80f) const { return lo > 0x1p-40f && hi < 0x1p40f && nlo > min_dividend && nhi < 0x1p80f; };
 };
 
 }  // namespace

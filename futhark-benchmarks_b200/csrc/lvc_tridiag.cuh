@@ -305,6 +305,7 @@ __device__ __forceinline__ void tri_row_step(TriRow& f, RangeCheck& in, float a,
     f.c1 = tri_mul(f.c1, l1);
     const float yp = tri_add(f.c0, tri_mul(f.c1, f.y0));
     in.divisor(p);
+    in.large(num);  // infinite where m1 s2 or m1 s3 overflows: bp is then too, not the NaN that near_div makes of it
     in.divisor(den);
     in.divisor(bp);
     in.dividend(a);
