@@ -60,8 +60,10 @@ struct RangeCheck {
     nlo = fminf(nlo, x == 0.0f ? 1.0f : fabsf(x));
     large(x);
   }
-  // min_dividend: where quotients are dividends in turn
-  __device__ __forceinline__ bool ok(float min_dividend = 0x1p-80f) const { return lo > 0x1p-40f && hi < 0x1p40f && nlo > min_dividend && nhi < 0x1p80f; };
+  // the dividends' limits: closer to one where quotients are dividends in turn
+  __device__ __forceinline__ bool ok(float least = 0x1p-80f, float most = 0x1p80f) const {
+    return lo > 0x1p-40f && hi < 0x1p40f && nlo > least && nhi < most;
+  }
 };
 
 }  // namespace

@@ -595,13 +595,14 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
             s1 = n1;
             s2 = n2;
             s3 = n3;
-            const float den = A_(M_(s2, b0), s3);
-            bp = near_div(A_(M_(s0, b0), s1), den, near_rcp(den));
+            const float num = A_(M_(s0, b0), s1), den = A_(M_(s2, b0), s3);
+            bp = near_div(num, den, near_rcp(den));
             const float l1 = S_(0.0f, near_div(a_[zz], bprev, rbprev));
             r0 = A_(d_[zz], M_(l1, r0));
             r1 = M_(r1, l1);
             yp = A_(r0, M_(r1, y0));
             in.divisor(pz);
+            in.large(num);  // infinite where m1 s2 or m1 s3 overflows
             in.divisor(den);
           }
           const float rb = near_rcp(bp);
@@ -690,7 +691,8 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
       __syncwarp();  // the next iteration refills this chunk's stage
     }
     cp_async_wait_all();
-    return !inner || in.ok(0x1p-60f);
+    // a_ and c_, quotients by dz or half of it, stay within 2^+-80
+    return !inner || in.ok(0x1p-60f, 0x1p59f);
   };
   if (!__all_sync(kAll, forward(std::true_type()))) forward(std::false_type());  // again, for any values
   float r0, r1;
