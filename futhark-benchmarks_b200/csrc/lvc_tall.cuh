@@ -90,6 +90,8 @@ LVC_HD TallLayout tall_layout(int X, int Ycs, int C) {
 }
 
 // ---- tensor memory: one lane of a warp's quarter per thread ----
+// All of these are .sync.aligned: the lanes of a warp arrive together.  After a branch
+// or a loop that lanes leave differently a barrier sees to that.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst, int ncols) {  // whole warp
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(dst)), "r"(ncols)
                : "memory");
@@ -159,6 +161,7 @@ __global__ void __launch_bounds__(32 * kTallWarps, 1) lvc_line_tall_kernel(Rollb
     mbar_init(barB, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
+  __syncwarp();
   if (warp == 0) {
     tmem_alloc(s_taddr, kCols);
     tmem_relinquish();
@@ -265,6 +268,7 @@ __global__ void __launch_bounds__(32 * kTallWarps, 1) lvc_line_tall_kernel(Rollb
         out_m = jy;
       }
     }
+    __syncthreads();  // after issue_copies and out_h (a __syncwarp at either place spills 24 bytes more)
     // Batch b of a step's pivots, unit b % 2 of round b / 2: loaded, and later stored.
     double2 pv[K / 2];
     double rb0[R];  // 1/b' of the column before unit 0's first, by round
@@ -479,9 +483,9 @@ __global__ void __launch_bounds__(32 * kTallWarps, 1) lvc_line_tall_kernel(Rollb
       if (more) {
         piv_store(0);
         piv_load(k - 1, 1);
+        issue_copies(k - 1, (sc + 1) & 1);  // into the table that the step before has read
       }
       __syncthreads();
-      if (more) issue_copies(k - 1, (sc + 1) & 1);
       if (clustered) {
         for (int col = tid; col < X; col += NT) {
           const int cg2 = col >> 6, w = col & 63;
