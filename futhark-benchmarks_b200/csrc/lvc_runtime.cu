@@ -776,11 +776,15 @@ template <typename S>
 int precision_of() { return sizeof(S) == sizeof(double) ? LVC_F64 : LVC_F32_STATE; }
 
 // The configuration of an X x Y grid: the context's tuned shape, else the
-// built-in choice (pad == false: without padding, for a caller short of memory).
+// built-in choice.  pad == false, for a caller short of memory: neither a tuned
+// nor a built-in shape that pads the grid.
 template <typename S>
 Config choose_config(const futhark_context* ctx, int X, int Y, bool pad = true, int outer = 0) {
   auto it = ctx->shapes.find(TuneKey{X, Y, precision_of<S>()});
-  if (it != ctx->shapes.end()) return it->second.cf;
+  if (it != ctx->shapes.end()) {
+    const Config& cf = it->second.cf;
+    if (pad || (tab_cols(cf, X) == X && tab_rows(cf, Y) == Y)) return cf;
+  }
   return pad ? default_config<S>(X, Y, ctx->max_smem, outer) : unpadded_config<S>(X, Y, ctx->max_smem);
 }
 
@@ -2128,14 +2132,11 @@ NoallocCarve noalloc_carve(const Config& cf, int outer, int numX, int numY, int 
 }
 
 // The shape the no-allocation entry point runs: the context's choice, or, when
-// its padded tables do not fit the static scratch and nothing is pinned, the
-// shape without padding.
+// its padded tables do not fit the static scratch, one without padding.
 Config noalloc_config(const futhark_context* ctx, int outer, int numX, int numY, int numT) {
   const Config cf = choose_config<double>(ctx, numX, numY, /*pad=*/true, outer);
-  if (!cf.pair || noalloc_carve(cf, outer, numX, numY, numT).need <= kNoAllocScratchBytes ||
-      ctx->shapes.count(TuneKey{numX, numY, LVC_F64}))
-    return cf;
-  return unpadded_config<double>(numX, numY, ctx->max_smem);
+  if (!cf.pair || noalloc_carve(cf, outer, numX, numY, numT).need <= kNoAllocScratchBytes) return cf;
+  return choose_config<double>(ctx, numX, numY, /*pad=*/false);
 }
 
 extern "C" int64_t lvc_entry_main_f64_noalloc_bytes(struct futhark_context* ctx, const int32_t outer,
