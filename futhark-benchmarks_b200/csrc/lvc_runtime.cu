@@ -2558,9 +2558,9 @@ bool server_admit(lvc_server* S, std::unique_lock<std::mutex>& lk) {
     if (e == cudaSuccess) e = cudaEventRecord(b->done, st);
   }
   lk.lock();
-  if (rc == FUTHARK_OUT_OF_MEMORY && (!S->inflight.empty() || take.size() > 1)) {
-    // the budget is taken by running batches (or fragmented): retry with
-    // fewer requests, or when running batches complete
+  if (rc == FUTHARK_OUT_OF_MEMORY && (!S->inflight.empty() || take.size() > 1 || !S->plan_lru.empty())) {
+    // the budget is taken by running batches (or fragmented): retry when running
+    // batches complete, without the idle plans, or with fewer requests
     if (P) plan_release(P);
     // the taken requests go back in arrival order
     auto requeue = [&]() {
@@ -2572,6 +2572,16 @@ bool server_admit(lvc_server* S, std::unique_lock<std::mutex>& lk) {
     };
     requeue();
     S->stream_busy[si] = false;
+    if (S->inflight.empty() && !S->plan_lru.empty()) {
+      // the idle plans split the room that is left
+      for (const auto& victim : S->plan_lru) {
+        auto& v = S->plan_cache[victim.first];
+        v.erase(std::find(v.begin(), v.end(), victim.second));
+        plan_release(victim.second);
+      }
+      S->plan_lru.clear();
+      return true;
+    }
     if (S->inflight.empty()) {
       // back off to half the batch; completed batches restore it (server_retire)
       S->cfg.max_batch_requests = std::max<int32_t>(1, (int32_t)take.size() / 2);
