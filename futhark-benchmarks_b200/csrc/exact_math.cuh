@@ -10,8 +10,9 @@
 // correctly rounded value: near_rcp was compared with __frcp_rn at every float of
 // exponent -125 .. 124, near_sqrt with __fsqrt_rn at every one of -87 .. 87,
 // near_div with __fdiv_rn at every pair of significands (2^46), without a
-// difference; scaling by powers of two changes nothing while no operand, quotient
-// or residual leaves the normal range.  The caller sees to that: it gathers the
+// difference (tests/test_gpu_exact_math.py repeats the first two and a sample of the
+// third); scaling by powers of two changes nothing while no operand, quotient or
+// residual leaves the normal range.  The caller sees to that: it gathers the
 // operands' range (RangeCheck) and starts over with __frcp_rn, __fdiv_rn and
 // __fsqrt_rn where it was left.
 //
