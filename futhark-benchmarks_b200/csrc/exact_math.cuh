@@ -61,6 +61,8 @@ struct RangeCheck {
     nlo = fminf(nlo, x == 0.0f ? 1.0f : fabsf(x));
     large(x);
   }
+  // where the divisors are near_rcp's alone
+  __device__ __forceinline__ bool reciprocals_ok() const { return lo >= 0x1p-125f && hi < 0x1p125f; }
   // the dividends' limits: closer to one where quotients are dividends in turn
   __device__ __forceinline__ bool ok(float least = 0x1p-80f, float most = 0x1p80f) const {
     return lo > 0x1p-40f && hi < 0x1p40f && nlo > least && nhi < most;

@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(32) lvc_tridag_row_kernel(int64_t rows, int m,
       if (m > 1) f.yn = py[m - 1];
     }
   }
-  if (__any_sync(0xffffffffu, !in.ok())) {  // again, for any values
+  if (__any_sync(0xffffffffu, FORM == 0 ? !in.reciprocals_ok() : !in.ok())) {  // again, for any values
     for (int q = 2; q < 4; q++)
 #pragma unroll 8
       for (int e = lane; e < n; e += 32) S[q * A + (ld == m ? e : e / m * ld + e % m)] = src(q)[e];

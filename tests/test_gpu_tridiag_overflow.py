@@ -53,3 +53,15 @@ def test_overflow_inside_and_nan_inputs(ctx, oracle):
         a[r, i], c[r, i - 1] = -(2.0**78), 2.0**55
     b[5, 3] = y[9, 0] = a[17, 18] = np.nan
     solve(ctx, oracle, (a, b, c, y))
+
+
+@pytest.mark.parametrize("form,oform", [("seq", "seq"), ("par", "par4")])
+@pytest.mark.parametrize("m", [7, 20, 115])
+def test_matrices_of_any_scale(ctx, oracle, m, form, oform):
+    rows = 64
+    a, b, c, y = (v.copy() for v in wl.tridiag_inputs(rows, m, seed=m))
+    for r in range(rows):  # pivots from below the normal floats to their upper end
+        s = np.float32(2.0 ** (-128 + 4 * r))
+        a[r], b[r], c[r] = a[r] * s, b[r] * s, c[r] * s
+    with np.errstate(all="ignore"):
+        assert same(ctx.tridag(a, b, c, y, form=form), oracle.tridag(a, b, c, y, form=oform))
