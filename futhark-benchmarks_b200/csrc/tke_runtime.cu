@@ -484,6 +484,17 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
     float s0 = 1.0f, s1 = 0.0f, s2 = 0.0f, s3 = 1.0f, b0 = 0.0f, y0 = 0.0f, r0 = 0.0f, r1 = 1.0f;
     float dm = 0.0f, cprev = 0.0f;
     double rbpprev = 0.0;         // 1 / b' of z - 1 (DR_)
+    // (near) y' and b' of the chunk before, the least |y'| in it but zeros
+    float ylast[kColCh], blast[kColCh], ymin = 1.0f;
+    // y'/b' of chunk k again where y' have faded out of near_div's range
+    auto small_quotients = [&](int k) {
+      if (!inner || ymin > 0x1p-80f) return;
+#pragma unroll
+      for (int zz = 0; zz < kColCh; zz++) {
+        const int z = k * kColCh + zz;
+        if (z < Z) (VEC ? qv[(int64_t)k * 8 * qs + zz] : q0[(int64_t)z * qs]) = __fdiv_rn(ylast[zz], blast[zz]);
+      }
+    };
     float bprev = 1.0f, rbprev = 1.0f;  // b' of z - 1 and its reciprocal (near_div)
     stage(0);
     cp_async_commit();
@@ -515,6 +526,8 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
         const float rdz_l = near_rcp(dz_l);
         in.divisor(M_(dz_l, dz_l));
         if (k + 1 < nch) ld_consts(k + 1);
+        if (k > 0) small_quotients(k - 1);
+        ymin = 1.0f;
         // (A) for the chunk's four z, independent of one another and of (B);
         // selections instead of branches
         float a_[kColCh], b_[kColCh], c_[kColCh], d_[kColCh];
@@ -541,6 +554,17 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
           }
         }
         fk[kColCh] = field(nxt, 1, 0);
+        float root[kColCh], tmin = 1.0f;
+#pragma unroll
+        for (int zz = 0; zz < kColCh; zz++) {
+          const float t0 = max_(0.0f, ft[zz]);
+          tmin = fminf(tmin, t0 == 0.0f ? 1.0f : t0);
+          root[zz] = near_sqrt(t0);
+        }
+        if (tmin < 0x1p-80f) {
+#pragma unroll
+          for (int zz = 0; zz < kColCh; zz++) root[zz] = __fsqrt_rn(max_(0.0f, ft[zz]));
+        }
         float v0[kColCh], v1[kColCh];
 #pragma unroll
         for (int zz = 0; zz < kColCh; zz++) {
@@ -553,7 +577,7 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
           const float d0 = z < Z - 1 ? M_(fac, A_(fk[zz], fk[zz + 1])) : 0.0f;  // delta (:103-108)
           const bool edge = land && z == ks, water = land && z >= ks;
           const float mx = water ? fm[zz] : 1.0f;
-          const float t0 = max_(0.0f, t), sq = near_sqrt(t0);
+          const float t0 = max_(0.0f, t), sq = root[zz];
           a_[zz] = !edge && water && z > 0 ? near_div(-dm, dd, rdd) : 0.0f;
           // 1 + (delta of the levels around) / dz + dissipation: the edge has
           // only the level above, the top only the one below and half a dz
@@ -569,7 +593,7 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
           dm = d0;
           if (VEC || zz < zn) {
             in.divisor(mx);
-            in.dividend(t0);
+            in.large(t0);
             in.dividend(d0);
           }
         }
@@ -607,7 +631,10 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
           }
           const float rb = near_rcp(bp);
           in.divisor(bp);
-          in.dividend(yp);
+          in.large(yp);
+          ymin = fminf(ymin, yp == 0.0f ? 1.0f : fabsf(yp));
+          ylast[zz] = yp;
+          blast[zz] = bp;
           cprev = c_[zz];
           bprev = bp;
           rbprev = rb;
@@ -691,6 +718,7 @@ __global__ void __launch_bounds__(kColWarps * 32, 4) tke_column_kernel(TkeArgs p
       __syncwarp();  // the next iteration refills this chunk's stage
     }
     cp_async_wait_all();
+    if constexpr (kNear) small_quotients(nch - 1);
     // a_ and c_, quotients by dz or half of it, stay within 2^+-80
     return !inner || in.ok(0x1p-60f, 0x1p59f);
   };
