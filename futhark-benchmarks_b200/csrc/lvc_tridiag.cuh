@@ -276,9 +276,11 @@ __device__ __forceinline__ void tri_row_element(TriRow& f, int i, int m, float a
 }
 
 // The same for i > 0 with near_rcp and near_div, exact while `in` holds.
-// FORM 1: c_i is not wanted at i == m - 1, and f.yn is y_i's new value there.
+// FORM 1: c_i is not wanted at i == m - 1, and f.yn is y_i's new value there.  y' is
+// left in yp, and in ymin the least but zeros, which `in` does not see from below.
 template <int FORM>
-__device__ __forceinline__ void tri_row_step(TriRow& f, RangeCheck& in, float a, float b, float& c, float& y) {
+__device__ __forceinline__ void tri_row_step(TriRow& f, RangeCheck& in, float a, float b, float& c, float& y,
+                                             float& yp, float& ymin) {
   if constexpr (FORM == 0) {
     const float d = tri_sub(b, tri_mul(a, f.cp));
     in.divisor(d);
@@ -303,20 +305,33 @@ __device__ __forceinline__ void tri_row_step(TriRow& f, RangeCheck& in, float a,
     const float l1 = tri_sub(0.0f, near_div(a, f.bp, f.rb));
     f.c0 = tri_add(y, tri_mul(l1, f.c0));
     f.c1 = tri_mul(f.c1, l1);
-    const float yp = tri_add(f.c0, tri_mul(f.c1, f.y0));
+    yp = tri_add(f.c0, tri_mul(f.c1, f.y0));
     in.divisor(p);
     in.large(num);  // infinite where m1 s2 or m1 s3 overflows: bp is then too, not the NaN that near_div makes of it
     in.divisor(den);
     in.divisor(bp);
     in.dividend(a);
     in.dividend(c);
-    in.dividend(yp);
+    in.large(yp);
+    ymin = fminf(ymin, yp == 0.0f ? 1.0f : fabsf(yp));
     f.cprev = c;
     f.bp = bp;
     f.rb = rb;
     y = yp == 0.0f ? tri_mul(yp, rb) : near_div(yp, bp, rb);
     c = tri_sub(0.0f, near_div(c, bp, rb));
   }
+}
+
+// y'/b' of elements first - 1 (y, b) and first .. first + n - 1 but a row's first, by
+// exact division.  Out of line, for rows in which y' fade out.
+static __device__ __noinline__ void tri_row_quotients(float* py, int first, int n, float y, float b, float4 y0, float4 y4,
+                                                      float4 b0, float4 b4) {
+  const float ys[kTriRowWin] = {y0.x, y0.y, y0.z, y0.w, y4.x, y4.y, y4.z, y4.w};
+  const float bs[kTriRowWin] = {b0.x, b0.y, b0.z, b0.w, b4.x, b4.y, b4.z, b4.w};
+  if (first > 0) py[first - 1] = tri_div(y, b);
+#pragma unroll
+  for (int k = 0; k < kTriRowWin; k++)
+    if (k < n && first + k > 0) py[first + k] = tri_div(ys[k], bs[k]);
 }
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
@@ -406,6 +421,7 @@ __global__ void __launch_bounds__(32) lvc_tridag_row_kernel(int64_t rows, int m,
   TriRow f;
   RangeCheck in;
   if (act) {
+    float ymin = 1.0f;
     float va[kTriRowWin], vb[kTriRowWin], vc[kTriRowWin], vy[kTriRowWin];
 #pragma unroll
     for (int k = 0; k < kTriRowWin; k += VW) {
@@ -420,10 +436,29 @@ __global__ void __launch_bounds__(32) lvc_tridag_row_kernel(int64_t rows, int m,
     const int full = m / kTriRowWin;
     const float *qa = pa, *qb = pb;
     float *qc = pc, *qy = py;
+    // FORM 1: quotients y'/b' whose y' have faded out of near_div's range are off the
+    // chain and taken again, a window's when the last element of it has been issued
+    // (which goes with the next window: its y' is not awaited).  57600 x 115 with y of
+    // 1e-30: 76 us, against 182 where such tiles take the exact pass below -- as they do
+    // with m = 4 k + 2, where the test makes ordinary systems 2 to 3 % slower (50000 x 50
+    // 20.8 and 21.5 us; otherwise they take the same time).
+    constexpr bool kLate = FORM == 1 && VW != 2;
+    float yq[kTriRowWin] = {}, bq[kTriRowWin] = {}, ylast = 0.0f, blast = 1.0f;
+    auto small_quotients = [&](int first, int n) {  // elements first - 1 .. first + n - 1
+      tri_row_quotients(py, first, n, ylast, blast, make_float4(yq[0], yq[1], yq[2], yq[3]),
+                        make_float4(yq[4], yq[5], yq[6], yq[7]), make_float4(bq[0], bq[1], bq[2], bq[3]),
+                        make_float4(bq[4], bq[5], bq[6], bq[7]));
+    };
     for (int w = 0; w < full; w++) {
+      float seen = 1.0f;
 #pragma unroll
       for (int k = 0; k < kTriRowWin; k++) {
-        if (k > 0 || w > 0) tri_row_step<FORM>(f, in, va[k], vb[k], vc[k], vy[k]);
+        if (kLate && k == kTriRowWin - 1) {
+          seen = ymin;
+          ymin = 1.0f;
+        }
+        if (k > 0 || w > 0) tri_row_step<FORM>(f, in, va[k], vb[k], vc[k], vy[k], yq[k], ymin);
+        bq[k] = f.bp;
         if (k % VW == VW - 1) {
           tri_row_store<VW>(qc, k - (VW - 1), vc);
           tri_row_store<VW>(qy, k - (VW - 1), vy);
@@ -433,6 +468,9 @@ __global__ void __launch_bounds__(32) lvc_tridag_row_kernel(int64_t rows, int m,
           tri_row_load<VW>(qy + kTriRowWin, k - (VW - 1), vy);
         }
       }
+      if (kLate && seen <= 0x1p-80f) small_quotients(w * kTriRowWin, kTriRowWin - 1);
+      ylast = yq[kTriRowWin - 1];
+      blast = bq[kTriRowWin - 1];
       qa += kTriRowWin;
       qb += kTriRowWin;
       qc += kTriRowWin;
@@ -442,11 +480,14 @@ __global__ void __launch_bounds__(32) lvc_tridag_row_kernel(int64_t rows, int m,
     for (int k = 0; k < kTriRowWin; k++) {
       if (full * kTriRowWin + k < m) {
         if (FORM == 1 && full * kTriRowWin + k == m - 1) vc[k] = 1.0f;
-        if (k > 0 || full > 0) tri_row_step<FORM>(f, in, va[k], vb[k], vc[k], vy[k]);
+        if (k > 0 || full > 0) tri_row_step<FORM>(f, in, va[k], vb[k], vc[k], vy[k], yq[k], ymin);
+        bq[k] = f.bp;
         qc[k] = vc[k];
         qy[k] = vy[k];
       }
     }
+    if (kLate && ymin <= 0x1p-80f) small_quotients(full * kTriRowWin, m - full * kTriRowWin);
+    if (!kLate && ymin <= 0x1p-80f) in.divisor(0.0f);  // out of range
     if constexpr (FORM == 1) {
       if (m > 1) f.yn = py[m - 1];
     }
