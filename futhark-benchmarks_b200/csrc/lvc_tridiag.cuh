@@ -322,6 +322,50 @@ __device__ __forceinline__ void tri_row_step(TriRow& f, RangeCheck& in, float a,
   }
 }
 
+template <int FORM>
+__device__ __forceinline__ bool tri_row_ok(const RangeCheck& in) {
+  return FORM == 0 ? in.reciprocals_ok() : in.ok();
+}
+
+// The forward pass for any values, an element at a time: by the fast divisions where
+// they hold for it, by exact ones where not.  A batch waits for a tile that comes here,
+// and in most rows that do a pivot or two is out of range: with one singular row
+// 57600 x 115 take 67 us (FORM 1) and 40 (FORM 0), by exact division throughout 74 and
+// 42, without it 49 and 36.  Out of line: in line ordinary systems of some lengths take
+// 1 to 3 % longer (50000 x 50 21.5 us against 20.7).
+template <int FORM>
+static __device__ __noinline__ TriRow tri_row_again(int m, const float* pa, const float* pb, float* pc, float* py) {
+  TriRow f;
+#pragma unroll 1
+  for (int i = 0; i < m; i++) {
+    const float a = pa[i], b = pb[i];
+    float c = pc[i], y = py[i];
+    RangeCheck in;
+    if constexpr (FORM == 1) {
+      in.divisor(f.bp);  // this element divides by it,
+      in.large(f.s2);    // and takes s2 to be finite
+    }
+    bool fast = i > 0 && tri_row_ok<FORM>(in);
+    if (fast) {
+      TriRow g = f;
+      float cg = FORM == 1 && i == m - 1 ? 1.0f : c, yg = y, yp = 0.0f, ymin = 1.0f;
+      tri_row_step<FORM>(g, in, a, b, cg, yg, yp, ymin);
+      fast = tri_row_ok<FORM>(in);
+      if (fast) {
+        f = g;
+        c = cg;
+        if (ymin <= 0x1p-80f) yg = tri_div(yp, g.bp);
+        if (FORM == 1 && i == m - 1) f.yn = yg;
+        y = yg;
+      }
+    }
+    if (!fast) tri_row_element<FORM>(f, i, m, a, b, c, y);
+    pc[i] = c;
+    py[i] = y;
+  }
+  return f;
+}
+
 // y'/b' of elements first - 1 (y, b) and first .. first + n - 1 but a row's first, by
 // exact division.  Out of line, for rows in which y' fade out.
 static __device__ __noinline__ void tri_row_quotients(float* py, int first, int n, float y, float b, float4 y0, float4 y4,
@@ -492,16 +536,12 @@ __global__ void __launch_bounds__(32) lvc_tridag_row_kernel(int64_t rows, int m,
       if (m > 1) f.yn = py[m - 1];
     }
   }
-  if (__any_sync(0xffffffffu, FORM == 0 ? !in.reciprocals_ok() : !in.ok())) {  // again, for any values
+  if (__any_sync(0xffffffffu, !tri_row_ok<FORM>(in))) {  // again, c and y copied in once more
     for (int q = 2; q < 4; q++)
 #pragma unroll 8
       for (int e = lane; e < n; e += 32) S[q * A + (ld == m ? e : e / m * ld + e % m)] = src(q)[e];
     __syncwarp();
-    f = TriRow();
-    if (act) {
-#pragma unroll 1
-      for (int i = 0; i < m; i++) tri_row_element<FORM>(f, i, m, pa[i], pb[i], pc[i], py[i]);
-    }
+    if (act) f = tri_row_again<FORM>(m, pa, pb, pc, py);
   }
 
   // backward, the solution in place of y, the same way from the end
