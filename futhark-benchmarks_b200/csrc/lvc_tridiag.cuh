@@ -328,13 +328,14 @@ __device__ __forceinline__ bool tri_row_ok(const RangeCheck& in) {
 }
 
 // The forward pass for any values, an element at a time: by the fast divisions where
-// they hold for it, by exact ones where not.  A batch waits for a tile that comes here,
-// and in most rows that do a pivot or two is out of range: with one singular row
-// 57600 x 115 take 67 us (FORM 1) and 40 (FORM 0), by exact division throughout 74 and
-// 42, without it 49 and 36.  Out of line: in line ordinary systems of some lengths take
-// 1 to 3 % longer (50000 x 50 21.5 us against 20.7).
+// they hold for it, by exact ones where not; returns yp or yn, which the backward fold
+// starts from.  A batch waits for a tile that comes here, and in most rows that do a
+// pivot or two is out of range: with one singular row 57600 x 115 take 67 us (FORM 1)
+// and 40 (FORM 0), by exact division throughout 74 and 42, without it 49 and 36.  Out of
+// line: in line ordinary systems of some lengths take 1 to 3 % longer (50000 x 50 21.5
+// us against 20.7).
 template <int FORM>
-static __device__ __noinline__ TriRow tri_row_again(int m, const float* pa, const float* pb, float* pc, float* py) {
+static __device__ __noinline__ float tri_row_again(int m, const float* pa, const float* pb, float* pc, float* py) {
   TriRow f;
 #pragma unroll 1
   for (int i = 0; i < m; i++) {
@@ -363,7 +364,7 @@ static __device__ __noinline__ TriRow tri_row_again(int m, const float* pa, cons
     pc[i] = c;
     py[i] = y;
   }
-  return f;
+  return FORM == 0 ? f.yp : f.yn;
 }
 
 // y'/b' of elements first - 1 (y, b) and first .. first + n - 1 but a row's first, by
@@ -536,16 +537,28 @@ __global__ void __launch_bounds__(32) lvc_tridag_row_kernel(int64_t rows, int m,
       if (m > 1) f.yn = py[m - 1];
     }
   }
+  float start = FORM == 0 ? f.yp : f.yn;  // of the backward fold
   if (__any_sync(0xffffffffu, !tri_row_ok<FORM>(in))) {  // again, c and y copied in once more
     for (int q = 2; q < 4; q++)
 #pragma unroll 8
       for (int e = lane; e < n; e += 32) S[q * A + (ld == m ? e : e / m * ld + e % m)] = src(q)[e];
     __syncwarp();
-    if (act) f = tri_row_again<FORM>(m, pa, pb, pc, py);
+    if constexpr (FORM == 1 && VW == 4) {
+      // exact division throughout: beside the other, ordinary systems take up to 3 %
+      // longer here (8000 x 200 23.7 us against 23.0)
+      f = TriRow();
+      if (act) {
+#pragma unroll 1
+        for (int i = 0; i < m; i++) tri_row_element<FORM>(f, i, m, pa[i], pb[i], pc[i], py[i]);
+      }
+      start = f.yn;
+    } else {
+      if (act) start = tri_row_again<FORM>(m, pa, pb, pc, py);
+    }
   }
 
   // backward, the solution in place of y, the same way from the end
-  float x = f.yp, c0 = 0.0f, c1 = 1.0f;
+  float x = start, c0 = 0.0f, c1 = 1.0f;
   auto back = [&](float p, float q) {  // p, q: the intermediates in c's and y's places
     if constexpr (FORM == 0) {
       x = tri_sub(q, tri_mul(p, x));  // x_i = yp_i - cp_i x_{i+1}  (:92-95)
@@ -553,16 +566,16 @@ __global__ void __launch_bounds__(32) lvc_tridag_row_kernel(int64_t rows, int m,
     } else {
       c0 = tri_add(q, tri_mul(p, c0));
       c1 = tri_mul(c1, p);
-      return tri_add(c0, tri_mul(c1, f.yn));
+      return tri_add(c0, tri_mul(c1, start));
     }
   };
   if (act) {
     const int wb = (m - 1) / kTriRowWin;  // whole windows before m - 1
     // element m - 1 (FORM 1: the fold's start, l0 = 0, l1 = 1), then the others of its window
-    float yl = f.yp;
+    float yl = start;
     if constexpr (FORM == 1) {
       c0 = tri_add(0.0f, tri_mul(1.0f, c0));
-      yl = tri_add(c0, tri_mul(c1, f.yn));
+      yl = tri_add(c0, tri_mul(c1, start));
     }
     py[m - 1] = yl;
     for (int i = m - 2; i >= wb * kTriRowWin; i--) py[i] = back(pc[i], py[i]);
