@@ -47,7 +47,7 @@ F_ALG = 77
 # state precision, from an ncu capture of those launches (the profile named
 # beside each figure); bench.py scales it by the step's option-cell-steps.
 TRAFFIC_PER_CELL_STEP = {
-    "f64": (2.027e9 / 4.496e9, "profiles/lvc_rollback_dram_mix64.txt"),
+    "f64": (1.983e9 / 4.496e9, "profiles/lvc_rollback_dram_mix64.txt"),
 }
 CALIB_DEV_BYTES = 112  # sizeof(lvc::CalibDev) (static_assert in lvc_layout.h), uploaded per calibration per step
 

@@ -686,7 +686,8 @@ double pair_cost(const Config& cf, int X, int Y, int outer) {
 // 50 x 50 8.4 against 21; 3 x 3 3.1 against 3.2, 200 x 7 16.5 against 15.3.
 // outer: the strikes of a call that runs alone (the entry points), 0 for batches
 // and serving, where the shape -- and with it the last bits of a price -- may not
-// depend on what a calibration is batched with.  There whole tiles keep the
+// depend on what a calibration is batched with (but for plans that device memory
+// does not hold padded, plan_new_locked).  There whole tiles keep the
 // smallest cluster: among other launch classes two small CTAs per SM are worth
 // less than they are alone (the 512-calibration mix takes 254.5 ms with 128 x 128,
 // 128 x 256 and 64 x 256 in the smallest clusters and 267 in ones of CTAs of 4096

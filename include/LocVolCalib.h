@@ -137,7 +137,9 @@ enum { LVC_F64 = 0, LVC_F32_STATE = 1 };
 
 /* A batch plan: the device tables, work lists and captured CUDA graph for a
  * fixed list of calibrations.  Prices of calibration c are at offset
- * sum_{c' < c} outer[c'] of the price vector. */
+ * sum_{c' < c} outer[c'] of the price vector.  Where device memory does not
+ * hold the plan with its grids padded to whole tiles, it is built with none of
+ * them padded (lvc_plan_shape tells): other kernels, other last bits. */
 struct lvc_plan;
 
 LVC_API int lvc_plan_new(struct futhark_context *ctx, const struct lvc_calibration *calibs, int32_t n,
@@ -312,7 +314,8 @@ LVC_API int lvc_shape_candidates(struct futhark_context *ctx, int32_t numX, int3
                                  int32_t precision, struct lvc_shape *out, int32_t max,
                                  int32_t *count);
 /* Pins a shape (matched on family, cluster and hbm_state) for a grid class;
- * NULL returns the class to the built-in choice. */
+ * NULL returns the class to the built-in choice.  A shape that pads the grid
+ * gives way to one that does not where the padded tables do not fit. */
 LVC_API int lvc_tuning_set(struct futhark_context *ctx, int32_t numX, int32_t numY,
                            int32_t precision, const struct lvc_shape *shape);
 /* The shape calibration `calib` of a plan runs under (FUTHARK_PROGRAM_ERROR
